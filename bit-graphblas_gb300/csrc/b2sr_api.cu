@@ -497,12 +497,13 @@ static b2sr_status run_rowbin(const b2sr_matrix* m_const, const float* x, float*
     Scratch fallback;
     st = matrix_scratch(m, s, rowbin_scratch_bytes(m->rowbin, m->T, 4), &partials, fallback);
     if (st != B2SR_SUCCESS) return st;
-    // T >= 16: only the set columns' x elements by default (R-MAT s20: 0.28 vs
-    // 0.34 ms at T = 16, 0.69 vs 1.04 ms at T = 32 on GB300).  T <= 8: whole x
-    // segments through the texture path by default (measured faster there);
-    // ld.global when asked for or when x cannot back a texture.
+    // T = 32: only set columns' x elements, whatever is asked for (whole
+    // segments: 1.04 vs 0.69 ms, R-MAT s20).  T = 16: those by default (0.28 vs
+    // 0.34 ms).  T <= 8: whole x segments through the texture path by default
+    // (measured faster there); ld.global when asked for or when x cannot back
+    // a texture.
     const int gather = m->shapes[B2SR_BIN_FULL_FULL].gather;
-    const bool sparse = gather == 3 || (gather == 0 && m->T >= 16);
+    const bool sparse = m->T == 32 || gather == 3 || (gather == 0 && m->T == 16);
     const cudaTextureObject_t xtex = (!sparse && gather != 1) ? vector_texture(x, sizeof(float) * (size_t)m->ncols) : 0;
     return rowbin_spmv(m->rowbin, view_of(m), x, y, accumulate, partials, xtex, sparse, s);
 }
@@ -1159,7 +1160,8 @@ b2sr_status b2sr_spmv_multi_bits(const b2sr_matrix* m_const, const void* d_x, vo
     Scratch fallback;
     st = matrix_scratch(m, s, rowbin_scratch_bytes(m->rowbin, m->T, word_bits / 8), &partials, fallback);
     if (st != B2SR_SUCCESS) return st;
-    const cudaTextureObject_t xtex = m->shapes[B2SR_BIN_FULL_FULL].gather != 1
+    // T >= 16 reads only set columns' words
+    const cudaTextureObject_t xtex = m->T <= 8 && m->shapes[B2SR_BIN_FULL_FULL].gather != 1
                                          ? vector_texture(d_x, (size_t)word_bits / 8 * (size_t)m->ncols) : 0;
     return rowbin_multi_bits(m->rowbin, view_of(m), d_x, d_y, d_mask, word_bits, accumulate, partials, xtex, s);
 }

@@ -59,6 +59,7 @@ struct RowBinPlan {
     int4* d_long = nullptr;
     int ntasks = 0, nlong = 0, nslots = 0;
     int nlong_short = 0;  // long rows with few slots, listed first in d_long
+    bool wide = false;    // T = 32: tasks of 128 tiles, for the staged FP32 form
     int task_off[7] = {0, 0, 0, 0, 0, 0, 0};
     int warp_off[7] = {0, 0, 0, 0, 0, 0, 0};
 };

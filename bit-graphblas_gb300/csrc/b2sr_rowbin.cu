@@ -1,12 +1,13 @@
-// Row-binned bin_full_full multiply: the fast path of y = A.x for packed
-// matrices (the merge-path kernel in b2sr_spmv_impl.cuh serves the other
-// variants and the reference-compatible shims).
+// Row-binned multiplies: the fast path of y = A.x for packed matrices.  The
+// forms below take a tile per lane; b2sr_widetile.cuh has those that spread a
+// 16 x 16 or 32 x 32 tile over lanes, on the same plan.
 //
 // Plan (once per matrix, built on the host from rowptr): every tile-row is
 // put in a bin by its tile count m; a bin fixes the group size G (lanes per
 // tile-row) so that each lane handles at most U tiles:
 //     m <= U -> G = 1,  m <= 2U -> 2,  ... ,  m <= 16U -> 16,  else G = 32.
-// Tile-rows longer than 32*U tiles are cut into segments of 32*U tiles.
+// Tile-rows longer than rb_seg tiles (32*U, mostly) are cut into segments of
+// that many.
 // A task is (row, first tile, end tile, out): out = -1 writes y directly,
 // out >= 0 writes a segment partial that the fix-up kernel adds in segment
 // order.  Tasks are stored bin by bin; a warp takes 32/G tasks of one bin.
@@ -26,20 +27,32 @@
 #include <vector>
 
 #include "b2sr_spmv_impl.cuh"
+#include "b2sr_widetile.cuh"
 
 namespace b2sr {
 
 constexpr int RB_BINS = 6;  // G = 1, 2, 4, 8, 16, 32
 
-template <int T> struct RowBinU { static constexpr int value = T <= 8 ? 4 : T == 16 ? 2 : 1; };
-// Tiles per lane of the bit-vector kernel's long-row tasks (a full warp
-// each, one step): 8 at T = 4, where its tiles need few registers.  The FP32 /
-// OR kernel keeps RowBinU there too (its registers buy occupancy), so the two
-// kernels have separate plans.
-constexpr int rb_long_u(int T) { return T == 4 ? 8 : T == 8 ? 4 : T == 16 ? 2 : 1; }
+// Tiles of a row that one lane of its group takes.
+__host__ __device__ constexpr int rb_u(int T) { return T <= 8 ? 4 : T == 16 ? 2 : 1; }
+// Rows of bin b that one warp takes.
+__host__ __device__ constexpr int rb_per_warp(int b) { return 32 >> b; }
+// Tiles of a long-row task: a full warp, one step of rb_u tiles a lane, or 8 a
+// lane for bit vectors at T = 4, where tiles need few registers (so at T = 4
+// the value and the bit kernels have a plan each).  At T = 32 four times as
+// many once the tiles are well past what L2 holds (WIDE_TILES of 132 bytes):
+// then the FP32 sums take the staged form of b2sr_widetile.cuh, which walks a
+// task in steps (R-MAT scale 20: 668 / 547 / 505 us with tasks of 32 / 64 /
+// 128); below, the lane-per-tile form is as fast or faster (R-MAT scale 16:
+// 33 against 40 us).
+constexpr int WIDE_TILES = 1 << 20;
+__host__ __device__ constexpr int rb_seg(int T, bool bits, int nt) {
+    return 32 * (T == 4 && bits ? 8 : T == 32 && nt >= WIDE_TILES ? 4 : rb_u(T));
+}
 template <int T, int G> struct RowBinTaskU {
-    static constexpr int value = G == 32 ? rb_long_u(T) : RowBinU<T>::value;
+    static constexpr int value = T == 4 && G == 32 ? 8 : rb_u(T);
 };
+constexpr int RB_BLOCK_WARPS = 2;  // warps per block of the value kernels
 
 struct RowBinArgs {
     const int* colind;
@@ -235,17 +248,30 @@ struct SparseColTile {
     }
 };
 
-// Register cap of the FP32 T = 8 dense and T = 32 set-column kernels and of
-// the 64-frontier OR kernel at T = 4 (255: none; the FP32 T = 4 and 16 forms
-// are capped through their launch bounds).  The 64-frontier cap: 36 warps per
-// SM instead of 34 at 60 registers; R-MAT scale 18 with 64 frontiers 53.5
-// instead of 61.4 us per call (48 spilled and took 58.9).
+// The value kernels' forms: FP32 sums take a lane per tile at T <= 16 (whole x
+// segments, or with SPARSE the set columns only) and at T = 32 with SPARSE;
+// the rest spread a tile over lanes (b2sr_widetile.cuh).
+template <int T, class Sem, bool SPARSE>
+constexpr bool RB_WIDE = std::is_same<Sem, SemSumF32>::value ? (T == 32 && !SPARSE) : T >= 16;
+
+// Register caps, for occupancy at the price of a few bytes of spills (255:
+// none; the FP32 T = 4 forms are capped through their launch bounds).  R-MAT
+// scale 20: FP32 T = 8 whole segments at 56 (36 warps per SM instead of 32 at
+// 63; 139 instead of 143 us, 48 was slower), T = 16 set columns at 64 (32
+// warps instead of 28 at 72; 264 instead of 278 us), T = 32 set columns at 80
+// (24 warps instead of 20 at 86; 645 instead of 690 us).  64-frontier OR at
+// T = 4: 56 (36 warps instead of 34 at 60; R-MAT scale 18 53.5 instead of 61.4
+// us per call, 48 spilled and took 58.9).  Wide tiles: 72, and 112 with 64-bit
+// values, do not lower the occupancy that the staged tiles' shared memory
+// allows.
 template <int T, class Sem, bool SPARSE> struct RowBinMaxReg {
     static constexpr bool f32 = std::is_same<Sem, SemSumF32>::value;
-    static constexpr int value = (f32 && T == 8 && !SPARSE)                       ? 56
-                                 : (f32 && T == 32 && SPARSE)                      ? 80
+    static constexpr int value = RB_WIDE<T, Sem, SPARSE>                          ? (sizeof(typename Sem::V) == 8 ? 112 : 72)
+                                 : (f32 && T == 8 && !SPARSE)                     ? 56
+                                 : (f32 && T == 16 && SPARSE)                     ? 64
+                                 : (f32 && T == 32)                               ? 80
                                  : (T == 4 && std::is_same<Sem, SemOrU64>::value) ? 56
-                                                                                   : 255;
+                                                                                  : 255;
 };
 
 template <int T, class Sem, bool SPARSE>
@@ -295,7 +321,7 @@ template <int T, class Sem, int G, bool SPARSE>
 __device__ __forceinline__ void rowbin_group(const RowBinArgs& a, int task, bool valid, int l) {
     using W = typename TileWord<T>::type;
     using V = typename Sem::V;
-    constexpr int U = RowBinU<T>::value;
+    constexpr int U = rb_u(T);
     const int4 t = valid ? __ldg(a.tasks + task) : make_int4(0, 0, 0, -2);
     const W* tiles = static_cast<const W*>(a.tiles);
     const V* x = static_cast<const V*>(a.x);
@@ -353,19 +379,22 @@ __device__ __forceinline__ void rowbin_group(const RowBinArgs& a, int task, bool
     }
 }
 
-template <int T, class Sem, bool SPARSE>
+// The rows of a warp in bin b, G = 1 << b: up to G * rb_u(T) tiles each, two
+// passes of tile slots.
+template <int T, class Sem, int G>
+__device__ __forceinline__ void wide_rows(const RowBinArgs& a, int task0, int tend) {
+    constexpr int SLOTS = G * rb_u(T), NT = WIDE_PASS<T> / SLOTS;
+    static_assert(2 * NT * G == 32, "two passes take the warp's 32 / G rows");
+#pragma unroll 1
+    for (int p = 0; p < 2; ++p) wide_group<T, Sem, SLOTS>(a, task0 + p * NT, tend);
+}
+
 // T = 4 with 32-bit values fits 32 registers, so 64 warps fit on an SM (90 us
-// instead of 102 us for R-MAT scale 20).  Register caps that buy occupancy
-// for a few bytes of spills, R-MAT scale 20: the FP32 T = 8 form at 56 (36
-// warps per SM instead of 32 at 63; 139 instead of 143 us, while 48 was
-// slower), the T = 16 set-column form at 64 (32 warps instead of 28 at 72;
-// 264 instead of 278 us) and the T = 32 set-column form at 80 (24 warps
-// instead of 20 at 86; 645 instead of 690 us; 72 spilled 356 bytes and was
-// slower).  Launched as two-warp blocks: 87 us instead of 90 us with 8-warp
-// blocks at T = 4, 143 us instead of 155 us at T = 8.
-__global__ void __launch_bounds__(256, (T == 4 && sizeof(typename Sem::V) == 4) ? (SPARSE ? 5 : 8)
-                                       : (T == 16 && SPARSE)                    ? 4
-                                                                                : 1)
+// instead of 102 us for R-MAT scale 20).  Launched as two-warp blocks: 87 us
+// instead of 90 us with 8-warp blocks at T = 4, 143 us instead of 155 us at
+// T = 8.
+template <int T, class Sem, bool SPARSE>
+__global__ void __launch_bounds__(256, (T == 4 && sizeof(typename Sem::V) == 4) ? (SPARSE ? 5 : 8) : 1)
     __maxnreg__((RowBinMaxReg<T, Sem, SPARSE>::value)) rowbin_spmv_kernel(RowBinArgs a) {
     const int warp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     const int lane = threadIdx.x & 31;
@@ -383,17 +412,29 @@ __global__ void __launch_bounds__(256, (T == 4 && sizeof(typename Sem::V) == 4) 
         }
     }
     const int b = RB_BINS - 1 - k;  // plan slot k holds bin RB_BINS-1-k
-    const int per_warp = 32 >> b;  // tasks per warp in bin b (G = 1 << b)
-    const int task = toff + (warp - woff) * per_warp + (lane >> b);
-    const bool valid = task < tend;
-    const int l = lane & ((1 << b) - 1);
-    switch (b) {
-        case 0: rowbin_group<T, Sem, 1, SPARSE>(a, task, valid, l); break;
-        case 1: rowbin_group<T, Sem, 2, SPARSE>(a, task, valid, l); break;
-        case 2: rowbin_group<T, Sem, 4, SPARSE>(a, task, valid, l); break;
-        case 3: rowbin_group<T, Sem, 8, SPARSE>(a, task, valid, l); break;
-        case 4: rowbin_group<T, Sem, 16, SPARSE>(a, task, valid, l); break;
-        default: rowbin_group<T, Sem, 32, SPARSE>(a, task, valid, l); break;
+    const int task0 = toff + (warp - woff) * rb_per_warp(b);  // the warp's first task (G = 1 << b lanes or slots each)
+    if constexpr (RB_WIDE<T, Sem, SPARSE>) {
+        __shared__ WideStage<T, typename Sem::V> stage[RB_BLOCK_WARPS];
+        switch (b) {
+            case 0: wide_rows<T, Sem, 1>(a, task0, tend); break;
+            case 1: wide_rows<T, Sem, 2>(a, task0, tend); break;
+            case 2: wide_rows<T, Sem, 4>(a, task0, tend); break;
+            case 3: wide_rows<T, Sem, 8>(a, task0, tend); break;
+            case 4: wide_rows<T, Sem, 16>(a, task0, tend); break;
+            default: wide_long<T, Sem>(a, task0, stage[threadIdx.x >> 5]); break;
+        }
+    } else {
+        const int task = task0 + (lane >> b);
+        const bool valid = task < tend;
+        const int l = lane & ((1 << b) - 1);
+        switch (b) {
+            case 0: rowbin_group<T, Sem, 1, SPARSE>(a, task, valid, l); break;
+            case 1: rowbin_group<T, Sem, 2, SPARSE>(a, task, valid, l); break;
+            case 2: rowbin_group<T, Sem, 4, SPARSE>(a, task, valid, l); break;
+            case 3: rowbin_group<T, Sem, 8, SPARSE>(a, task, valid, l); break;
+            case 4: rowbin_group<T, Sem, 16, SPARSE>(a, task, valid, l); break;
+            default: rowbin_group<T, Sem, 32, SPARSE>(a, task, valid, l); break;
+        }
     }
 }
 
@@ -482,10 +523,8 @@ struct RowBinPlanHost {
     int nslots = 0;
 };
 
-static RowBinPlanHost build_rowbin_plan(const std::vector<int>& rowptr, int T, int UL) {
-    const int U = T <= 8 ? 4 : T == 16 ? 2 : 1;
-    const int nb = (int)rowptr.size() - 1;
-    const int seg = 32 * UL;
+static RowBinPlanHost build_rowbin_plan(const std::vector<int>& rowptr, int T, bool bits) {
+    const int U = rb_u(T), nb = (int)rowptr.size() - 1, seg = rb_seg(T, bits, rowptr[nb]);
     std::vector<std::vector<int4>> bins(RB_BINS);
     RowBinPlanHost p;
     for (int i = 0; i < nb; ++i) {
@@ -515,7 +554,7 @@ static RowBinPlanHost build_rowbin_plan(const std::vector<int>& rowptr, int T, i
         const int b = RB_BINS - 1 - k;
         p.tasks.insert(p.tasks.end(), bins[b].begin(), bins[b].end());
         p.task_off[k + 1] = (int)p.tasks.size();
-        const int per_warp = 32 >> b;
+        const int per_warp = rb_per_warp(b);
         p.warp_off[k + 1] = p.warp_off[k] + ((int)bins[b].size() + per_warp - 1) / per_warp;
     }
     return p;
@@ -529,12 +568,13 @@ b2sr_status rowbin_plan_create(const int* d_rowptr, int nb, int T, bool bits, Ro
         set_cuda_error(e);
         return B2SR_ERR_CUDA;
     }
-    RowBinPlanHost h = build_rowbin_plan(rp, T, bits ? rb_long_u(T) : (T <= 8 ? 4 : T == 16 ? 2 : 1));
+    RowBinPlanHost h = build_rowbin_plan(rp, T, bits);
     RowBinPlan p;
     p.ntasks = (int)h.tasks.size();
     p.nlong = (int)h.long_rows.size();
     p.nlong_short = h.nlong_short;
     p.nslots = h.nslots;
+    p.wide = T == 32 && rp[nb] >= WIDE_TILES;
     for (int b = 0; b <= RB_BINS; ++b) {
         p.task_off[b] = h.task_off[b];
         p.warp_off[b] = h.warp_off[b];
@@ -595,11 +635,13 @@ static b2sr_status run_rowbin(const RowBinPlan& p, const MatView& A, const void*
     if (warps > 0) {
         kernel_timer_mark(s, true);
         // two-warp blocks: finer scheduling
+        constexpr int W = RB_BLOCK_WARPS;
+        const unsigned blocks = (unsigned)((warps + W - 1) / W);
         if constexpr (std::is_same<Sem, SemSumF32>::value) {
-            if (sparse) rowbin_spmv_kernel<T, Sem, true><<<(warps + 1) / 2, 64, 0, s>>>(a);
-            else rowbin_spmv_kernel<T, Sem, false><<<(warps + 1) / 2, 64, 0, s>>>(a);
+            if (T == 32 ? !p.wide : sparse) rowbin_spmv_kernel<T, Sem, true><<<blocks, 32 * W, 0, s>>>(a);
+            else rowbin_spmv_kernel<T, Sem, false><<<blocks, 32 * W, 0, s>>>(a);
         } else {
-            rowbin_spmv_kernel<T, Sem, false><<<(warps + 1) / 2, 64, 0, s>>>(a);
+            rowbin_spmv_kernel<T, Sem, false><<<blocks, 32 * W, 0, s>>>(a);
         }
         kernel_timer_mark(s, false);
         B2SR_LAUNCH_CHECK();
@@ -660,6 +702,7 @@ struct RowBinBitsArgs {
     void* partials;  // long-row segment slots: one word (KIND 0/1) or T ints (KIND 2/3)
     int task_off[RB_BINS + 1];
     int warp_off[RB_BINS + 1];
+    int nbc;  // x words (0: x is not read)
     int accumulate;
     const int* push_ctl;  // auto direction: the push kernel's counters (null: always pull)
     int push_pct;
@@ -750,12 +793,18 @@ __device__ __forceinline__ void bits_group(const RowBinBitsArgs& a, int task, bo
     }
 }
 
+template <int T, int KIND, int G>
+__device__ __forceinline__ void wide_bits_rows(const RowBinBitsArgs& a, int task0, int tend, bool skip) {
+#pragma unroll 1
+    for (int p = 0; p < 2; ++p) wide_bits_group<T, KIND, G>(a, task0 + p * (WIDE_PASS<T> / G), tend, skip);
+}
+
 // T <= 8 fits 32 registers: 64 warps per SM.  So do the T = 16 bit kernels
 // (bin_bin_bin, masked) without spills: 64 warps per SM instead of 48 at 40,
-// R-MAT scale 20 121.5 instead of 133.1 us per call (the count kinds and
-// T = 32 spill at such caps).
+// R-MAT scale 20 121.5 instead of 133.1 us per call (the count kinds spill at
+// such a cap).  T = 32 fits 40: 48 warps.
 template <int T, int KIND>
-__global__ void __launch_bounds__(256, T <= 8 ? 8 : 1) __maxnreg__((T == 16 && KIND <= 1 ? 32 : 255))
+__global__ void __launch_bounds__(256, T <= 8 ? 8 : 1) __maxnreg__((T == 32 ? 40 : T == 16 && KIND <= 1 ? 32 : 255))
     rowbin_bits_kernel(RowBinBitsArgs a) {
     const int warp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     const int lane = threadIdx.x & 31;
@@ -771,17 +820,29 @@ __global__ void __launch_bounds__(256, T <= 8 ? 8 : 1) __maxnreg__((T == 16 && K
         }
     }
     const int b = RB_BINS - 1 - k;  // plan slot k holds bin RB_BINS-1-k
-    const int per_warp = 32 >> b;
-    const int task = toff + (warp - woff) * per_warp + (lane >> b);
-    const bool valid = task < tend;
-    const int l = lane & ((1 << b) - 1);
-    switch (b) {
-        case 0: bits_group<T, KIND, 1>(a, task, valid, l); break;
-        case 1: bits_group<T, KIND, 2>(a, task, valid, l); break;
-        case 2: bits_group<T, KIND, 4>(a, task, valid, l); break;
-        case 3: bits_group<T, KIND, 8>(a, task, valid, l); break;
-        case 4: bits_group<T, KIND, 16>(a, task, valid, l); break;
-        default: bits_group<T, KIND, 32>(a, task, valid, l); break;
+    const int task0 = toff + (warp - woff) * rb_per_warp(b);
+    if constexpr (T == 32) {
+        const bool skip = mostly_zero(static_cast<const uint32_t*>(a.x), a.nbc);
+        switch (b) {
+            case 0: wide_bits_rows<T, KIND, 1>(a, task0, tend, skip); break;
+            case 1: wide_bits_rows<T, KIND, 2>(a, task0, tend, skip); break;
+            case 2: wide_bits_rows<T, KIND, 4>(a, task0, tend, skip); break;
+            case 3: wide_bits_rows<T, KIND, 8>(a, task0, tend, skip); break;
+            case 4: wide_bits_rows<T, KIND, 16>(a, task0, tend, skip); break;
+            default: wide_bits_long<T, KIND>(a, task0, skip); break;
+        }
+    } else {
+        const int task = task0 + (lane >> b);
+        const bool valid = task < tend;
+        const int l = lane & ((1 << b) - 1);
+        switch (b) {
+            case 0: bits_group<T, KIND, 1>(a, task, valid, l); break;
+            case 1: bits_group<T, KIND, 2>(a, task, valid, l); break;
+            case 2: bits_group<T, KIND, 4>(a, task, valid, l); break;
+            case 3: bits_group<T, KIND, 8>(a, task, valid, l); break;
+            case 4: bits_group<T, KIND, 16>(a, task, valid, l); break;
+            default: bits_group<T, KIND, 32>(a, task, valid, l); break;
+        }
     }
 }
 
@@ -892,6 +953,7 @@ static b2sr_status run_rowbin_bits(const RowBinPlan& p, const MatView& A, const 
         a.task_off[b] = p.task_off[b];
         a.warp_off[b] = p.warp_off[b];
     }
+    a.nbc = x ? (int)(((long long)A.ncols + T - 1) / T) : 0;
     a.accumulate = accumulate;
     a.push_ctl = link.ctl;
     a.push_pct = link.pct;
@@ -901,7 +963,7 @@ static b2sr_status run_rowbin_bits(const RowBinPlan& p, const MatView& A, const 
     const unsigned fix_blocks = (unsigned)((fixup_warps(p.nlong, p.nlong_short) + 7) / 8);
     if (link.ctl && link.gate) {
         // the pull is launched from the device only when it is chosen
-        const int wpb = T <= 8 ? 2 : 8;
+        const int wpb = T != 16 ? 2 : 8;
         B2SR_CUDA_TRY(launch_dependent(rowbin_bits_gate_kernel<T, KIND>, 1u, 32u, s, a,
                                        (unsigned)((warps + wpb - 1) / wpb), 32u * wpb, (const int4*)p.d_long,
                                        p.nlong, p.nlong_short, fix_blocks));
@@ -909,10 +971,10 @@ static b2sr_status run_rowbin_bits(const RowBinPlan& p, const MatView& A, const 
         return B2SR_SUCCESS;
     }
     if (warps > 0) {
-        // two-warp blocks at T <= 8 (finer scheduling: faster than 256-thread
-        // blocks), but eight-warp blocks behind an auto-direction push, where
-        // most blocks only retire
-        const int wpb = (T <= 8 && !link.ctl) ? 2 : 8;
+        // two-warp blocks (finer scheduling: faster than 256-thread blocks),
+        // but eight-warp blocks at T = 16, and behind an auto-direction push,
+        // where most blocks only retire
+        const int wpb = (T != 16 && !link.ctl) ? 2 : 8;
         if (timed) kernel_timer_mark(s, true);
         rowbin_bits_kernel<T, KIND><<<(warps + wpb - 1) / wpb, 32 * wpb, 0, s>>>(a);
         if (timed) kernel_timer_mark(s, false);
