@@ -653,37 +653,6 @@ static b2sr_status count_set_bits(b2sr_matrix* m, cudaStream_t s) {
     return st;
 }
 
-// Validate + count + scan into browptr (nb + 1 entries).  Returns the tile
-// count in *nt.  Synchronises `s`.
-static b2sr_status structure_pass(const int* rowptr, const int* colind, int nrows, int ncols,
-                                  int nnz, int T, int nb, int* browptr, int* nt, cudaStream_t s) {
-    int* flags = static_cast<int*>(dev_alloc(2 * sizeof(int)));
-    if (!flags) return B2SR_ERR_ALLOC;
-    b2sr_status st = B2SR_SUCCESS;
-    int h[3] = {0, 0, 0};
-    do {
-        if (nrows > 0) {
-            st = launch_validate_csr(rowptr, colind, nrows, ncols, nnz, flags, s);
-            if (st != B2SR_SUCCESS) break;
-            st = launch_count_tiles(rowptr, colind, nrows, nb, T, flags, browptr, s);
-            if (st != B2SR_SUCCESS) break;
-        } else {
-            cudaError_t e = cudaMemsetAsync(flags, 0, sizeof(int), s);
-            if (e != cudaSuccess) { set_cuda_error(e); st = B2SR_ERR_CUDA; break; }
-        }
-        st = launch_exclusive_scan(browptr, nb, flags + 1, s);  // synchronises s
-        if (st != B2SR_SUCCESS) break;
-        cudaError_t e = cudaMemcpy(h, flags, 2 * sizeof(int), cudaMemcpyDeviceToHost);
-        if (e == cudaSuccess) e = cudaMemcpy(h + 2, browptr + nb, sizeof(int), cudaMemcpyDeviceToHost);
-        if (e != cudaSuccess) { set_cuda_error(e); st = B2SR_ERR_CUDA; break; }
-        if (h[0] != 0) { st = B2SR_ERR_INVALID_CSR; break; }
-        if (h[1] != 0) { st = B2SR_ERR_OVERFLOW; break; }
-        *nt = h[2];
-    } while (0);
-    dev_free(flags);
-    return st;
-}
-
 // The shims' fast path.  A kernel-launch shim gets raw B2SR arrays on every
 // call, the way the reference drivers launch bmv{T}_* in their timed loops
 // (bmv_eval/test_bin_full_full.cu:285-297).  The first call on a set of arrays
@@ -822,24 +791,24 @@ b2sr_status b2sr_pack_csr(const int* d_rowptr, const int* d_colind, int nrows, i
     do {
         m->rowptr = static_cast<int*>(dev_alloc(sizeof(int) * ((size_t)m->nb + 1)));
         if (!m->rowptr) { st = B2SR_ERR_ALLOC; break; }
+        PackJob job;
         int nt = 0;
-        st = structure_pass(d_rowptr, d_colind, nrows, ncols, nnz, tile_dim, m->nb, m->rowptr, &nt, s);
+        st = job.count(d_rowptr, d_colind, nrows, ncols, nnz, tile_dim, m->rowptr, &nt, &m->nnz, s);
         if (st != B2SR_SUCCESS) break;
         m->nt = nt;
-        const size_t cbytes = padded_bytes(sizeof(int) * (size_t)nt);
-        const size_t tbytes = padded_bytes((size_t)nt * tile_dim * word_bytes(tile_dim));
-        m->colind = static_cast<int*>(dev_alloc(cbytes));
-        m->tiles = dev_alloc(tbytes);
+        // the fill writes every colind and tile word; only the padding is zeroed
+        const size_t cbytes = sizeof(int) * (size_t)nt, tbytes = (size_t)nt * tile_dim * word_bytes(tile_dim);
+        m->colind = static_cast<int*>(dev_alloc(padded_bytes(cbytes)));
+        m->tiles = dev_alloc(padded_bytes(tbytes));
         if (!m->colind || !m->tiles) { st = B2SR_ERR_ALLOC; break; }
-        cudaError_t e = cudaMemsetAsync(m->colind, 0, cbytes, s);
-        if (e == cudaSuccess) e = cudaMemsetAsync(m->tiles, 0, tbytes, s);
+        cudaError_t e = cudaMemsetAsync(reinterpret_cast<char*>(m->colind) + cbytes, 0, padded_bytes(cbytes) - cbytes, s);
+        if (e == cudaSuccess)
+            e = cudaMemsetAsync(static_cast<char*>(m->tiles) + tbytes, 0, padded_bytes(tbytes) - tbytes, s);
         if (e != cudaSuccess) { set_cuda_error(e); st = B2SR_ERR_CUDA; break; }
-        if (nt > 0) {
-            st = launch_fill_tiles(d_rowptr, d_colind, nrows, m->nb, tile_dim, m->rowptr, m->colind,
-                                   m->tiles, s);
-            if (st != B2SR_SUCCESS) break;
-        }
-        st = count_set_bits(m, s);
+        if (nt > 0) st = job.fill(m->colind, m->tiles);
+        if (st != B2SR_SUCCESS) break;
+        e = cudaStreamSynchronize(s);  // the matrix may be used on any stream from here on
+        if (e != cudaSuccess) { set_cuda_error(e); st = B2SR_ERR_CUDA; }
     } while (0);
     if (st != B2SR_SUCCESS) {
         cudaStreamSynchronize(s);
@@ -1233,9 +1202,9 @@ b2sr_status b2sr_ref_csr2bsr_nnz(const int* d_csrRowPtr, const int* d_csrColInd,
         set_cuda_error(e);
         return B2SR_ERR_CUDA;
     }
-    const int nb = (int)(((long long)nrows + blocksize - 1) / blocksize);
-    return structure_pass(d_csrRowPtr, d_csrColInd, nrows, ncols, nnz, blocksize, nb, d_bsrRowPtr,
-                          h_nblocks, nullptr);
+    if (nnz < 0) return B2SR_ERR_INVALID_CSR;
+    PackJob job;
+    return job.count(d_csrRowPtr, d_csrColInd, nrows, ncols, nnz, blocksize, d_bsrRowPtr, h_nblocks, nullptr, nullptr);
 }
 
 b2sr_status b2sr_ref_csr2bsr_batch(const int* h_csrRowPtr, const int* h_csrColInd, int nrows,
@@ -1256,19 +1225,17 @@ b2sr_status b2sr_ref_csr2bsr_batch(const int* h_csrRowPtr, const int* h_csrColIn
         if (e == cudaSuccess && nnz > 0)
             e = cudaMemcpy(d_ci, h_csrColInd, sizeof(int) * (size_t)nnz, cudaMemcpyHostToDevice);
         if (e != cudaSuccess) { set_cuda_error(e); st = B2SR_ERR_CUDA; break; }
-        // Re-derive the structure to check it against the caller's rowptr.
+        // Re-derive the structure to check it against the caller's tile count.
         int* chk = static_cast<int*>(dev_alloc(sizeof(int) * ((size_t)nblockrows + 1)));
         if (!chk) { st = B2SR_ERR_ALLOC; break; }
         int nt = 0;
-        st = structure_pass(d_rp, d_ci, nrows, ncols, nnz, blocksize, nblockrows, chk, &nt, nullptr);
+        PackJob job;
+        st = job.count(d_rp, d_ci, nrows, ncols, nnz, blocksize, chk, &nt, nullptr, nullptr);
         dev_free(chk);
         if (st != B2SR_SUCCESS) break;
         if (nt != nblocks) { st = B2SR_ERR_INVALID_VALUE; break; }
         if (nblocks > 0) {
-            e = cudaMemset(d_bsrVal, 0, (size_t)nblocks * blocksize * word_bytes(blocksize));
-            if (e != cudaSuccess) { set_cuda_error(e); st = B2SR_ERR_CUDA; break; }
-            st = launch_fill_tiles(d_rp, d_ci, nrows, nblockrows, blocksize, d_bsrRowPtr, d_bsrColInd,
-                                   d_bsrVal, nullptr);
+            st = job.fill(d_bsrColInd, d_bsrVal);
             if (st != B2SR_SUCCESS) break;
             e = cudaDeviceSynchronize();
             if (e != cudaSuccess) { set_cuda_error(e); st = B2SR_ERR_CUDA; break; }

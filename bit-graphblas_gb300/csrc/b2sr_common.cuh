@@ -189,18 +189,30 @@ inline cudaError_t launch_dependent(void (*kernel)(KArgs...), unsigned grid, uns
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // ---- packing (b2sr_pack.cu) ---------------------------------------------------
-// Device CSR validation; writes error bits into *d_flag (0 = valid).
-b2sr_status launch_validate_csr(const int* rowptr, const int* colind, int nrows, int ncols,
-                                int nnz, int* d_flag, cudaStream_t s);
-// Tiles per tile-row into d_counts[nb]; does nothing if *d_csr_flag != 0.
-b2sr_status launch_count_tiles(const int* rowptr, const int* colind, int nrows, int nb, int T,
-                               const int* d_csr_flag, int* d_counts, cudaStream_t s);
+// CSR -> B2SR in two passes with shared scratch.  count() validates the CSR,
+// writes browptr (nb + 1) and returns the number of tiles and of distinct
+// entries; it synchronizes the stream.  B2SR_ERR_INVALID_CSR: nothing is
+// packed.  fill() then writes colind (nt) and every tile word (nt * T), on the
+// same stream.  The scratch is freed, after the stream has drained, with the
+// object.
+class PackJob {
+public:
+    ~PackJob();
+    b2sr_status count(const int* rowptr, const int* colind, int nrows, int ncols, int nnz, int T, int* browptr, int* nt,
+                      long long* set_bits, cudaStream_t s);
+    b2sr_status fill(int* bcolind, void* tiles);
+    struct Layout;
+
+private:
+    void* scratch = nullptr;
+    cudaStream_t s = nullptr;
+    int T = 0, nb = 0;
+    long long max_chunks = 0, n_entries = 0;
+    bool wide = false;  // 64-bit sort keys
+};
 // In-place exclusive scan of d_vals[0..n) with the total written to d_vals[n].
 // d_vals must have n + 1 entries.  d_err receives 1 if the total overflows int32.
 b2sr_status launch_exclusive_scan(int* d_vals, int n, int* d_err, cudaStream_t s);
-// Fill colind/tiles from CSR given the B2SR rowptr.
-b2sr_status launch_fill_tiles(const int* rowptr, const int* colind, int nrows, int nb, int T,
-                              const int* browptr, int* bcolind, void* tiles, cudaStream_t s);
 b2sr_status launch_pack_vec_bits(const float* x, int n, int T, void* bits, cudaStream_t s);
 b2sr_status launch_unpack_vec_bits(const void* bits, int n, int T, float* out, cudaStream_t s);
 // Set bits of a B2SR matrix (for the descriptor); result in *d_count (int64).
