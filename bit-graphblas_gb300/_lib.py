@@ -64,6 +64,7 @@ _PROTOS = {
     "b2sr_last_cuda_error": (C.c_int, []),
     "b2sr_version": (C.c_int, []),
     "b2sr_set_allocator": (None, [ALLOC_FN, FREE_FN, c_void_p]),
+    "b2sr_trim": (None, []),
     "b2sr_pack_csr": (C.c_int, [c_void_p, c_void_p, C.c_int, C.c_int, C.c_int, C.c_int, c_void_p,
                                 C.POINTER(c_void_p)]),
     "b2sr_matrix_wrap": (C.c_int, [c_void_p, c_void_p, c_void_p, C.c_int, C.c_int, C.c_int, C.c_int,

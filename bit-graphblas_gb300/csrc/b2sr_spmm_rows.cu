@@ -538,7 +538,8 @@ b2sr_status spmm_rows_plan_create(const int* d_rowptr, const void* d_tiles, int 
         e = cudaGetLastError();
         if (e == cudaSuccess)
             e = cudaMemcpyAsync(rbits.data(), d_bits, sizeof(long long) * (size_t)nb, cudaMemcpyDeviceToHost, s);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+        const cudaError_t drained = cudaStreamSynchronize(s);
+        if (e == cudaSuccess) e = drained;
         dev_free(d_bits);
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);

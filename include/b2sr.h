@@ -84,11 +84,17 @@ int b2sr_last_cuda_error(void);
 int b2sr_version(void);  /* major*10000 + minor*100 + patch */
 
 /* Allocation hook: every device allocation the library makes goes through it
- * (NULL restores cudaMalloc/cudaFree).  Lets a caller route allocations into
- * its own pool and lets tests inject allocation failures. */
+ * (NULL restores the library's own).  Lets a caller route allocations into its
+ * own pool and lets tests inject allocation failures.  A block is given to
+ * free_fn only when no kernel of the library uses it any more. */
 typedef void* (*b2sr_alloc_fn)(size_t bytes, void* ctx);
 typedef void (*b2sr_free_fn)(void* ptr, void* ctx);
 void b2sr_set_allocator(b2sr_alloc_fn alloc_fn, b2sr_free_fn free_fn, void* ctx);
+
+/* Without a hook the library keeps up to 1/256 of a device's memory that it has
+ * freed, for its next allocations.  b2sr_trim gives all of it back to the
+ * driver (so does an allocation that would otherwise fail). */
+void b2sr_trim(void);
 
 /* ---- packing -------------------------------------------------------------- */
 /* CSR (int32, zero-based, column indices non-decreasing within each row;
