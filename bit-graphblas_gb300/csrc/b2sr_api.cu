@@ -441,30 +441,22 @@ static b2sr_status get_plan(const b2sr_matrix* m_const, b2sr_variant v, cudaStre
     return B2SR_SUCCESS;
 }
 
-// Row-binned plans of `m`, built on first use.
-// Plans are built from a host copy of rowptr (a synchronizing download), so
-// they cannot be built while `s` is being captured: a multiply made during
-// capture needs one made on the matrix before it (B2SR_ERR_NOT_SUPPORTED
-// otherwise).
-static b2sr_status ensure_rowbin(b2sr_matrix* m, cudaStream_t s) {
+// Row-binned plan of `m` for the value or the bit kernels, built on first use
+// (the same plan except at T = 4).  Building it waits for its totals, so it
+// cannot be built while `s` is being captured: a multiply made during capture
+// needs one made on the matrix before it (B2SR_ERR_NOT_SUPPORTED otherwise).
+static b2sr_status ensure_rowbin(b2sr_matrix* m, bool bits, const RowBinPlan** out, cudaStream_t s) {
+    bits = bits && m->T == 4;
+    RowBinPlan& plan = bits ? m->rowbin_bits : m->rowbin;
+    bool& ready = bits ? m->rowbin_bits_ready : m->rowbin_ready;
     std::lock_guard<std::mutex> lk(g_plan_mu);
-    if (!m->rowbin_ready) {
+    if (!ready) {
         if (stream_capturing(s)) return B2SR_ERR_NOT_SUPPORTED;
-        b2sr_status st = rowbin_plan_create(m->rowptr, m->nb, m->T, false, &m->rowbin, s);
+        b2sr_status st = rowbin_plan_create(m->rowptr, m->nb, m->nt, m->T, bits, &plan, s);
         if (st != B2SR_SUCCESS) return st;
-        m->rowbin_ready = true;
+        ready = true;
     }
-    return B2SR_SUCCESS;
-}
-
-static b2sr_status ensure_rowbin_bits(b2sr_matrix* m, cudaStream_t s) {
-    std::lock_guard<std::mutex> lk(g_plan_mu);
-    if (!m->rowbin_bits_ready) {
-        if (stream_capturing(s)) return B2SR_ERR_NOT_SUPPORTED;
-        b2sr_status st = rowbin_plan_create(m->rowptr, m->nb, m->T, true, &m->rowbin_bits, s);
-        if (st != B2SR_SUCCESS) return st;
-        m->rowbin_bits_ready = true;
-    }
+    *out = &plan;
     return B2SR_SUCCESS;
 }
 
@@ -520,11 +512,12 @@ static b2sr_status run_multiply(const b2sr_matrix* m, b2sr_variant v, const void
             }
         }
         b2sr_status st = B2SR_SUCCESS;
+        const RowBinPlan* plan = nullptr;
         if (dir != 2) {
-            st = ensure_rowbin_bits(mm, s);
+            st = ensure_rowbin(mm, true, &plan, s);
             if (st != B2SR_SUCCESS) return st;
         }
-        const size_t pull_bytes = dir == 2 ? 0 : (rowbin_bits_scratch_bytes(m->rowbin_bits, m->T) + 255) / 256 * 256;
+        const size_t pull_bytes = dir == 2 ? 0 : (rowbin_bits_scratch_bytes(*plan, m->T) + 255) / 256 * 256;
         void* scratch = nullptr;
         Scratch fallback;
         st = matrix_scratch(m, s, pull_bytes + (dir ? push_scratch_bytes(m->nbc, m->nt) : 0), &scratch, fallback);
@@ -556,7 +549,7 @@ static b2sr_status run_multiply(const b2sr_matrix* m, b2sr_variant v, const void
                 st = launch_direction_count(view_of(t), x, m->nt, as->state, hint_dev + kind, as->side);
                 if (st != B2SR_SUCCESS) return st;
                 B2SR_CUDA_TRY(cudaEventRecord(as->join, as->side));
-                st = rowbin_bits(m->rowbin_bits, view_of(m), kind, x, y, mask, accumulate, scratch, PushLink{}, true, s);
+                st = rowbin_bits(*plan, view_of(m), kind, x, y, mask, accumulate, scratch, PushLink{}, true, s);
                 B2SR_CUDA_TRY(cudaStreamWaitEvent(s, as->join, 0));
                 return st;
             }
@@ -567,7 +560,7 @@ static b2sr_status run_multiply(const b2sr_matrix* m, b2sr_variant v, const void
             if (st != B2SR_SUCCESS || dir == 2) return st;
             link.gate = hint != nullptr;
         }
-        st = rowbin_bits(m->rowbin_bits, view_of(m), kind, x, y, mask, accumulate, scratch, link, dir == 0, s);
+        st = rowbin_bits(*plan, view_of(m), kind, x, y, mask, accumulate, scratch, link, dir == 0, s);
         if (dir == 1) kernel_timer_mark(s, false);
         return st;
     }
@@ -592,11 +585,12 @@ static b2sr_status run_rowbin(const b2sr_matrix* m_const, const float* x, float*
     if (!m || !y || (!x && m->nt > 0)) return B2SR_ERR_INVALID_VALUE;
     if ((uintptr_t)x % 16 != 0 || (uintptr_t)y % 16 != 0) return B2SR_ERR_INVALID_VALUE;
     cudaStream_t s = as_stream(stream);
-    b2sr_status st = ensure_rowbin(m, s);
+    const RowBinPlan* plan = nullptr;
+    b2sr_status st = ensure_rowbin(m, false, &plan, s);
     if (st != B2SR_SUCCESS) return st;
     void* partials = nullptr;
     Scratch fallback;
-    st = matrix_scratch(m, s, rowbin_scratch_bytes(m->rowbin, m->T, 4), &partials, fallback);
+    st = matrix_scratch(m, s, rowbin_scratch_bytes(*plan, m->T, 4), &partials, fallback);
     if (st != B2SR_SUCCESS) return st;
     // T = 32: only set columns' x elements, whatever is asked for (whole
     // segments: 1.04 vs 0.69 ms, R-MAT s20).  T = 16: those by default (0.28 vs
@@ -606,7 +600,7 @@ static b2sr_status run_rowbin(const b2sr_matrix* m_const, const float* x, float*
     const int gather = m->shapes[B2SR_BIN_FULL_FULL].gather;
     const bool sparse = m->T == 32 || gather == 3 || (gather == 0 && m->T == 16);
     const cudaTextureObject_t xtex = (!sparse && gather != 1) ? vector_texture(x, sizeof(float) * (size_t)m->ncols) : 0;
-    return rowbin_spmv(m->rowbin, view_of(m), x, y, accumulate, partials, xtex, sparse, s);
+    return rowbin_spmv(*plan, view_of(m), x, y, accumulate, partials, xtex, sparse, s);
 }
 
 // Chunk starts of the SpMM work queue, built on first use.
@@ -653,7 +647,8 @@ static b2sr_status run_spmm_api(const b2sr_matrix* m, const V* X, int k, long lo
             std::lock_guard<std::mutex> lk(g_plan_mu);
             if (!mm->spmm_rows_ready) {
                 if (stream_capturing(s)) return B2SR_ERR_NOT_SUPPORTED;  // as ensure_rowbin
-                b2sr_status st = spmm_rows_plan_create(mm->rowptr, mm->tiles, mm->nb, mm->T, mm->num_sms, &mm->spmm_rows, s);
+                b2sr_status st = spmm_rows_plan_create(mm->rowptr, mm->tiles, mm->nb, mm->nt, mm->nnz, mm->T, mm->num_sms,
+                                                       &mm->spmm_rows, s);
                 if (st != B2SR_SUCCESS) return st;
                 mm->spmm_rows_ready = true;
             }
@@ -1236,16 +1231,17 @@ b2sr_status b2sr_spmv_multi_bits(const b2sr_matrix* m_const, const void* d_x, vo
         return B2SR_ERR_INVALID_VALUE;
     if (d_mask && accumulate) return B2SR_ERR_INVALID_VALUE;
     cudaStream_t s = as_stream(stream);
-    b2sr_status st = ensure_rowbin(m, s);
+    const RowBinPlan* plan = nullptr;
+    b2sr_status st = ensure_rowbin(m, false, &plan, s);
     if (st != B2SR_SUCCESS) return st;
     void* partials = nullptr;
     Scratch fallback;
-    st = matrix_scratch(m, s, rowbin_scratch_bytes(m->rowbin, m->T, word_bits / 8), &partials, fallback);
+    st = matrix_scratch(m, s, rowbin_scratch_bytes(*plan, m->T, word_bits / 8), &partials, fallback);
     if (st != B2SR_SUCCESS) return st;
     // T >= 16 reads only set columns' words
     const cudaTextureObject_t xtex = m->T <= 8 && m->shapes[B2SR_BIN_FULL_FULL].gather != 1
                                          ? vector_texture(d_x, (size_t)word_bits / 8 * (size_t)m->ncols) : 0;
-    return rowbin_multi_bits(m->rowbin, view_of(m), d_x, d_y, d_mask, word_bits, accumulate, partials, xtex, s);
+    return rowbin_multi_bits(*plan, view_of(m), d_x, d_y, d_mask, word_bits, accumulate, partials, xtex, s);
 }
 
 b2sr_status b2sr_spmv_bin_bin_bin_masked(const b2sr_matrix* m, const void* d_xbits,

@@ -213,6 +213,10 @@ private:
 // In-place exclusive scan of d_vals[0..n) with the total written to d_vals[n].
 // d_vals must have n + 1 entries.  d_err receives 1 if the total overflows int32.
 b2sr_status launch_exclusive_scan(int* d_vals, int n, int* d_err, cudaStream_t s);
+// The same without a wait: scratch of exclusive_scan_scratch(n) bytes, *d_err
+// left alone without an overflow.
+size_t exclusive_scan_scratch(long long n);
+void exclusive_scan_async(int* d_vals, int n, int* d_err, void* scratch, cudaStream_t s);
 b2sr_status launch_pack_vec_bits(const float* x, int n, int T, void* bits, cudaStream_t s);
 b2sr_status launch_unpack_vec_bits(const void* bits, int n, int T, float* out, cudaStream_t s);
 // Set bits of a B2SR matrix (for the descriptor); result in *d_count (int64).
@@ -226,6 +230,45 @@ b2sr_status launch_count_bits(const void* tiles, long long nwords, int T,
 // lies outside [0, nbc).
 b2sr_status launch_transpose(const int* rowptr, const int* colind, const void* tiles, int nb, int nbc, int nt, int T,
                              int* rowptr_t, int* colind_t, void* tiles_t, cudaStream_t s);
+
+// ---- task lists (b2sr_plan.cu) -----------------------------------------------------
+constexpr int PLAN_CLASSES = 64;
+// How tile-rows become tasks.  A tile-row of more than `seg` tiles is cut into
+// segments: of seg tiles (BINS), or near-equal ones (the others), which with
+// row_bits also hold at most about seg_bits set bits each.  Tasks are listed by
+// class, tile-rows ascending inside a class:
+//   BINS    nbins bins by tile count (bin b: up to unit << b tiles), the last
+//           bin first; long rows of at most narrow_slots slots listed first
+//   TWO     tasks of at least a quarter of seg, then the rest
+//   LENGTH  longest first, in four classes per octave
+//   BITS    most set bits first, in two classes per octave
+struct PlanRule {
+    enum Kind { BINS, TWO, LENGTH, BITS } kind;
+    int seg;
+    int classes;
+    int unit = 0, nbins = 0, narrow_slots = 0;
+    const long long* row_bits = nullptr;
+    long long seg_bits = 0;
+};
+struct PlanBounds {
+    long long tasks, longs, slots;
+};
+struct PlanOut {
+    int4* tasks;     // (tile-row, first tile, end tile, slot or -1)
+    int4* longs;     // (tile-row, first slot, slots, 0)
+    int* slot_long;  // long row of every slot (null: not wanted)
+    int* info;
+    int cap_tasks, cap_long, cap_slots;
+};
+struct PlanTotals {
+    int tasks = 0, longs = 0, narrow = 0, slots = 0;
+    int first[PLAN_CLASSES + 1] = {0};  // first task of every class, and their number
+};
+// Array sizes that hold the plan of a matrix with nt tiles and `bits` set bits.
+PlanBounds plan_bounds(const PlanRule& r, int nb, long long nt, long long bits);
+// Fills the arrays (of those sizes).  Synchronizes `s`.
+b2sr_status build_plan(const PlanRule& rule, const int* rowptr, int nb, const PlanBounds& cap, int4* tasks, int4* longs,
+                       int* slot_long, PlanTotals* totals, cudaStream_t s);
 
 // ---- multiply (b2sr_spmv.cu) --------------------------------------------------
 struct MatView {
@@ -262,10 +305,9 @@ size_t spmm_scratch_bytes(int T, int elem_bytes, int nchunks, int k);
 int spmm_grid_warps(int num_sms);
 
 // ---- row-task dense right-hand sides (b2sr_spmm_rows.cu) --------------------------
-// Synchronizes `s` (it reads rowptr, and at T = 16 / 32 each tile-row's set
-// bits, on the host).
-b2sr_status spmm_rows_plan_create(const int* d_rowptr, const void* d_tiles, int nb, int T, int num_sms,
-                                  SpmmRowsPlan* out, cudaStream_t s);
+// Synchronizes `s`.
+b2sr_status spmm_rows_plan_create(const int* d_rowptr, const void* d_tiles, int nb, int nt, long long nnz, int T,
+                                  int num_sms, SpmmRowsPlan* out, cudaStream_t s);
 void spmm_rows_plan_free(SpmmRowsPlan* p);
 size_t spmm_rows_scratch_bytes(const SpmmRowsPlan& p, int T, int elem_bytes, int k);
 size_t spmm_rows_state_bytes(const SpmmRowsPlan& p);
@@ -276,7 +318,7 @@ b2sr_status spmm_rows_launch(const MatView& A, const SpmmRowsPlan& p, const V* X
 
 // ---- row-binned bin_full_full (b2sr_rowbin.cu) ------------------------------------
 // bits: the plan of the bit-vector kernels (longer long-row tasks at T = 4).
-b2sr_status rowbin_plan_create(const int* d_rowptr, int nb, int T, bool bits, RowBinPlan* out, cudaStream_t s);
+b2sr_status rowbin_plan_create(const int* d_rowptr, int nb, int nt, int T, bool bits, RowBinPlan* out, cudaStream_t s);
 void rowbin_plan_free(RowBinPlan* p);
 size_t rowbin_scratch_bytes(const RowBinPlan& p, int T, int value_bytes);
 // Bit-vector variants on the same plan: kind 0 bin_bin_bin, 1 masked, 2 int32

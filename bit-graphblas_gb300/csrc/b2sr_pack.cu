@@ -559,10 +559,7 @@ size_t exclusive_scan_scratch(long long n) {
     return sizeof(long long) * (size_t)((n > 0 ? (n + SCAN_TILE - 1) / SCAN_TILE : 1) + 1);
 }
 
-// In-place exclusive scan of vals[0, n), total to vals[n]; scratch of
-// exclusive_scan_scratch(n) bytes; *err is set on overflow and left alone
-// otherwise.  Asynchronous.
-static void scan_async(int* vals, int n, int* err, void* scratch, cudaStream_t s) {
+void exclusive_scan_async(int* vals, int n, int* err, void* scratch, cudaStream_t s) {
     const int nblocks = n > 0 ? (n + SCAN_TILE - 1) / SCAN_TILE : 1;
     long long* partial = static_cast<long long*>(scratch);
     scan_reduce_kernel<<<nblocks, SCAN_THREADS, 0, s>>>(vals, n, partial);
@@ -574,7 +571,7 @@ b2sr_status launch_exclusive_scan(int* d_vals, int n, int* d_err, cudaStream_t s
     B2SR_CUDA_TRY(cudaMemsetAsync(d_err, 0, sizeof(int), s));
     void* partial = dev_alloc(exclusive_scan_scratch(n));
     if (!partial) return B2SR_ERR_ALLOC;
-    scan_async(d_vals, n, d_err, partial, s);
+    exclusive_scan_async(d_vals, n, d_err, partial, s);
     cudaError_t e = cudaGetLastError();
     // The scratch is freed after the stream drains: the caller synchronises the
     // stream right after the scan (it needs the total on the host).
@@ -678,7 +675,7 @@ b2sr_status PackJob::count(const int* rowptr, const int* colind, int nrows, int 
             validate_entries_kernel<false><<<blocks, 256, 0, s>>>(colind, ncols, nnz, l.starts, l.info);
     }
     chunk_plan_kernel<<<(nb + 255) / 256, 256, 0, s>>>(rowptr, nrows, nb, T, l.info, l.choff);
-    scan_async(l.choff, nb, &l.info->err, l.scan, s);
+    exclusive_scan_async(l.choff, nb, &l.info->err, l.scan, s);
     chunk_rows_kernel<<<(nb + 255) / 256, 256, 0, s>>>(l.choff, nb, (int)max_chunks, l.chunk_tr);
     const int blocks = (int)((max_chunks + 1 + PACK_WARPS - 1) / PACK_WARPS);
     switch (T) {
@@ -687,7 +684,7 @@ b2sr_status PackJob::count(const int* rowptr, const int* colind, int nrows, int 
         case 16: launch_sort<16>(wide, blocks, rowptr, colind, nrows, nb, l, (int)max_chunks, s); break;
         default: launch_sort<32>(wide, blocks, rowptr, colind, nrows, nb, l, (int)max_chunks, s); break;
     }
-    scan_async(l.coff, (int)max_chunks, &l.info->err, l.scan, s);
+    exclusive_scan_async(l.coff, (int)max_chunks, &l.info->err, l.scan, s);
     tile_rowptr_kernel<<<(nb + 1 + 255) / 256, 256, 0, s>>>(l.choff, l.coff, nb, browptr, l.info);
     B2SR_LAUNCH_CHECK();
     PackInfo h;

@@ -2,7 +2,7 @@
 // forms below take a tile per lane; b2sr_widetile.cuh has those that spread a
 // 16 x 16 or 32 x 32 tile over lanes, on the same plan.
 //
-// Plan (once per matrix, built on the host from rowptr): every tile-row is
+// Plan (once per matrix, b2sr_plan.cu): every tile-row is
 // put in a bin by its tile count m; a bin fixes the group size G (lanes per
 // tile-row) so that each lane handles at most U tiles:
 //     m <= U -> G = 1,  m <= 2U -> 2,  ... ,  m <= 16U -> 16,  else G = 32.
@@ -514,95 +514,38 @@ rowbin_fixup_kernel(const int4* __restrict__ long_rows, int nlong, int nshort,
 }
 
 // ---- plan -----------------------------------------------------------------------------
-struct RowBinPlanHost {
-    std::vector<int4> tasks;
-    std::vector<int4> long_rows;
-    int nlong_short = 0;
-    int task_off[RB_BINS + 1];
-    int warp_off[RB_BINS + 1];
-    int nslots = 0;
-};
-
-static RowBinPlanHost build_rowbin_plan(const std::vector<int>& rowptr, int T, bool bits) {
-    const int U = rb_u(T), nb = (int)rowptr.size() - 1, seg = rb_seg(T, bits, rowptr[nb]);
-    std::vector<std::vector<int4>> bins(RB_BINS);
-    RowBinPlanHost p;
-    for (int i = 0; i < nb; ++i) {
-        const int b0 = rowptr[i], m = rowptr[i + 1] - b0;
-        int b = 0;
-        while (b < RB_BINS - 1 && m > (U << b)) ++b;
-        if (m <= seg) {
-            bins[b].push_back(make_int4(i, b0, b0 + m, -1));
-        } else {
-            const int nseg = (m + seg - 1) / seg;
-            p.long_rows.push_back(make_int4(i, p.nslots, nseg, 0));
-            for (int s = 0; s < nseg; ++s)
-                bins[RB_BINS - 1].push_back(make_int4(i, b0 + s * seg, std::min(b0 + (s + 1) * seg, b0 + m),
-                                                      p.nslots + s));
-            p.nslots += nseg;
-        }
-    }
-    // long rows with at most FIX_G slots first (the fix-up's narrow groups)
-    std::stable_partition(p.long_rows.begin(), p.long_rows.end(), [](const int4& L) { return L.z <= FIX_G; });
-    p.nlong_short = (int)std::count_if(p.long_rows.begin(), p.long_rows.end(),
-                                       [](const int4& L) { return L.z <= FIX_G; });
-    // plan slot k holds bin RB_BINS-1-k: the long-row warps come first, so
-    // they start early and the short bins fill the tail
-    p.task_off[0] = 0;
-    p.warp_off[0] = 0;
-    for (int k = 0; k < RB_BINS; ++k) {
-        const int b = RB_BINS - 1 - k;
-        p.tasks.insert(p.tasks.end(), bins[b].begin(), bins[b].end());
-        p.task_off[k + 1] = (int)p.tasks.size();
-        const int per_warp = rb_per_warp(b);
-        p.warp_off[k + 1] = p.warp_off[k] + ((int)bins[b].size() + per_warp - 1) / per_warp;
-    }
-    return p;
-}
-
-b2sr_status rowbin_plan_create(const int* d_rowptr, int nb, int T, bool bits, RowBinPlan* out, cudaStream_t s) {
-    std::vector<int> rp((size_t)nb + 1);
-    cudaError_t e = cudaMemcpyAsync(rp.data(), d_rowptr, sizeof(int) * rp.size(), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (e != cudaSuccess) {
-        set_cuda_error(e);
-        return B2SR_ERR_CUDA;
-    }
-    RowBinPlanHost h = build_rowbin_plan(rp, T, bits);
+b2sr_status rowbin_plan_create(const int* d_rowptr, int nb, int nt, int T, bool bits, RowBinPlan* out, cudaStream_t s) {
+    // class k holds bin RB_BINS-1-k: the long-row warps come first, so they
+    // start early and the short bins fill the tail; long rows with at most
+    // FIX_G slots go first (the fix-up's narrow groups)
+    PlanRule rule{PlanRule::BINS, rb_seg(T, bits, nt), RB_BINS, rb_u(T), RB_BINS, FIX_G};
+    const PlanBounds cap = plan_bounds(rule, nb, nt, 0);
     RowBinPlan p;
-    p.ntasks = (int)h.tasks.size();
-    p.nlong = (int)h.long_rows.size();
-    p.nlong_short = h.nlong_short;
-    p.nslots = h.nslots;
-    p.wide = T == 32 && rp[nb] >= WIDE_TILES;
-    for (int b = 0; b <= RB_BINS; ++b) {
-        p.task_off[b] = h.task_off[b];
-        p.warp_off[b] = h.warp_off[b];
-    }
-    p.d_tasks = static_cast<int4*>(dev_alloc(sizeof(int4) * (size_t)std::max(p.ntasks, 1)));
-    p.d_long = static_cast<int4*>(dev_alloc(sizeof(int4) * (size_t)std::max(p.nlong, 1)));
-    if (!p.d_tasks || !p.d_long) {
+    p.d_tasks = static_cast<int4*>(dev_alloc(sizeof(int4) * (size_t)(cap.tasks + cap.longs)));
+    if (!p.d_tasks) return B2SR_ERR_ALLOC;
+    p.d_long = p.d_tasks + cap.tasks;
+    PlanTotals t;
+    const b2sr_status st = build_plan(rule, d_rowptr, nb, cap, p.d_tasks, p.d_long, nullptr, &t, s);
+    if (st != B2SR_SUCCESS) {
         dev_free(p.d_tasks);
-        dev_free(p.d_long);
-        return B2SR_ERR_ALLOC;
+        return st;
     }
-    e = cudaSuccess;
-    if (p.ntasks) e = cudaMemcpy(p.d_tasks, h.tasks.data(), sizeof(int4) * (size_t)p.ntasks, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess && p.nlong)
-        e = cudaMemcpy(p.d_long, h.long_rows.data(), sizeof(int4) * (size_t)p.nlong, cudaMemcpyHostToDevice);
-    if (e != cudaSuccess) {
-        set_cuda_error(e);
-        dev_free(p.d_tasks);
-        dev_free(p.d_long);
-        return B2SR_ERR_CUDA;
+    p.ntasks = t.tasks;
+    p.nlong = t.longs;
+    p.nlong_short = t.narrow;
+    p.nslots = t.slots;
+    p.wide = T == 32 && nt >= WIDE_TILES;
+    for (int k = 0; k <= RB_BINS; ++k) p.task_off[k] = t.first[k];
+    for (int k = 0; k < RB_BINS; ++k) {
+        const int per_warp = rb_per_warp(RB_BINS - 1 - k);
+        p.warp_off[k + 1] = p.warp_off[k] + (p.task_off[k + 1] - p.task_off[k] + per_warp - 1) / per_warp;
     }
     *out = p;
     return B2SR_SUCCESS;
 }
 
 void rowbin_plan_free(RowBinPlan* p) {
-    dev_free(p->d_tasks);
-    dev_free(p->d_long);
+    dev_free(p->d_tasks);  // d_long is part of it
     p->d_tasks = nullptr;
     p->d_long = nullptr;
 }

@@ -4,7 +4,7 @@
 // whole tile-row at T = 4 and 8, and one group of 8 of its rows at T = 16
 // and 32.
 //
-// Plan (host, once per matrix): one task per tile-row; a tile-row longer
+// Plan (once per matrix, b2sr_plan.cu): one task per tile-row; a tile-row longer
 // than spmm_rows_seg() tiles (a share of one resident warp's part of all the
 // tiles) is cut into near-equal segments whose partial rows go to slots.  The warp that finishes a row's last segment (a per-row
 // arrival counter) adds the row's slots in segment order and writes Y, so a
@@ -513,10 +513,18 @@ __global__ void tile_row_bits_kernel(const int* __restrict__ rowptr, const uint3
     }
 }
 
-b2sr_status spmm_rows_plan_create(const int* d_rowptr, const void* d_tiles, int nb, int T, int num_sms,
-                                  SpmmRowsPlan* out, cudaStream_t s) {
-    std::vector<int> rp((size_t)nb + 1);
-    cudaError_t e = cudaMemcpyAsync(rp.data(), d_rowptr, sizeof(int) * rp.size(), cudaMemcpyDeviceToHost, s);
+b2sr_status spmm_rows_plan_create(const int* d_rowptr, const void* d_tiles, int nb, int nt, long long nnz, int T,
+                                  int num_sms, SpmmRowsPlan* out, cudaStream_t s) {
+    // Queue order.  T = 4: tasks of at least a quarter of a segment first,
+    // then the rest, each class in tile-row order, so the queue ends on short
+    // tasks while tile-rows that share X rows (the blocks of a batched graph)
+    // still run together: R-MAT scale 18 / 20 as fast as longest first, and
+    // 512 stacked ER graphs 1.86 ms against 2.85 ms longest first (2.61 ms in
+    // row order with fixed segments).  T = 8: longest first (R-MAT scale 18:
+    // 0.233 against 0.268 ms with the split).  T = 16 / 32: most set bits
+    // first.
+    PlanRule rule{T == 4 ? PlanRule::TWO : T == 8 ? PlanRule::LENGTH : PlanRule::BITS, spmm_rows_seg(T, nt, num_sms),
+                  T == 4 ? 2 : PLAN_CLASSES};
     // T = 16 / 32: the set bits of every tile-row.  A row group holding hub
     // rows carries far more set bits than its tiles suggest (R-MAT scale 18,
     // T = 32: ~9.3 K X-row loads for one warp in a tile-bounded segment of
@@ -526,111 +534,44 @@ b2sr_status spmm_rows_plan_create(const int* d_rowptr, const void* d_tiles, int 
     // bits and the long rows reduced per row group: R-MAT scale 18, k = 64,
     // 0.295 / 0.377 ms at T = 16 / 32 against 0.484 / 1.027 ms with
     // tile-bounded segments).
-    const bool by_bits = T >= 16 && nb > 0;
-    std::vector<long long> rbits;
-    if (e == cudaSuccess && by_bits) {
-        long long* d_bits = static_cast<long long*>(dev_alloc(sizeof(long long) * (size_t)nb));
+    long long* d_bits = nullptr;
+    if (T >= 16 && nb > 0) {
+        d_bits = static_cast<long long*>(dev_alloc(sizeof(long long) * (size_t)nb));
         if (!d_bits) return B2SR_ERR_ALLOC;
-        rbits.resize((size_t)nb);
         const long long blocks = std::min<long long>(((long long)nb * 32 + 255) / 256, 65535LL * 8);
         tile_row_bits_kernel<<<(unsigned)blocks, 256, 0, s>>>(d_rowptr, static_cast<const uint32_t*>(d_tiles), nb,
                                                                 T * T / 32, d_bits);
-        e = cudaGetLastError();
-        if (e == cudaSuccess)
-            e = cudaMemcpyAsync(rbits.data(), d_bits, sizeof(long long) * (size_t)nb, cudaMemcpyDeviceToHost, s);
-        const cudaError_t drained = cudaStreamSynchronize(s);
-        if (e == cudaSuccess) e = drained;
-        dev_free(d_bits);
+        rule.row_bits = d_bits;
+        rule.seg_bits = std::max(1024LL, nnz / ((long long)std::max(num_sms, 1) * ROWS_BLOCKS<32> * ROWS_WARPS));
     }
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (e != cudaSuccess) {
-        set_cuda_error(e);
-        return B2SR_ERR_CUDA;
-    }
-    const int seg = spmm_rows_seg(T, rp[nb], num_sms);
-    long long seg_bits = 0;
-    if (by_bits) {
-        long long total = 0;
-        for (long long v : rbits) total += v;
-        const long long warps = (long long)std::max(num_sms, 1) * ROWS_BLOCKS<32> * ROWS_WARPS;
-        seg_bits = std::max(1024LL, total / warps);
-    }
-    std::vector<int4> tasks, longs;
-    std::vector<long long> work;  // estimated set bits of each task (T = 16 / 32)
-    tasks.reserve((size_t)nb + 16);
-    int nslots = 0;
-    for (int i = 0; i < nb; ++i) {
-        const int b0 = rp[i], m = rp[i + 1] - b0;
-        int nseg = (m + seg - 1) / seg;  // near-equal segments of at most seg tiles
-        if (by_bits) nseg = (int)std::min<long long>(m, std::max<long long>(nseg, (rbits[i] + seg_bits - 1) / seg_bits));
-        if (nseg <= 1) {
-            tasks.push_back(make_int4(i, b0, b0 + m, -1));
-            if (by_bits) work.push_back(rbits[i]);
-        } else {
-            longs.push_back(make_int4(i, nslots, nseg, 0));
-            for (int q = 0; q < nseg; ++q) {
-                const int t0 = b0 + (int)((long long)m * q / nseg), t1 = b0 + (int)((long long)m * (q + 1) / nseg);
-                tasks.push_back(make_int4(i, t0, t1, nslots + q));
-                if (by_bits) work.push_back((long long)((double)rbits[i] * (t1 - t0) / m));
-            }
-            nslots += nseg;
-        }
-    }
-    // Queue order.  T = 4: tasks of at least a quarter of a segment first,
-    // then the rest, each class in tile-row order, so the queue ends on short
-    // tasks while tile-rows that share X rows (the blocks of a batched graph)
-    // still run together: R-MAT scale 18 / 20 as fast as longest first, and
-    // 512 stacked ER graphs 1.86 ms against 2.85 ms longest first (2.61 ms in
-    // row order with fixed segments).  T = 8: longest first (R-MAT scale 18:
-    // 0.233 against 0.268 ms with the split).  T = 16 / 32: most set bits
-    // first.
-    if (by_bits) {
-        std::vector<int> order(tasks.size());
-        for (size_t q = 0; q < order.size(); ++q) order[q] = (int)q;
-        std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return work[x] > work[y]; });
-        std::vector<int4> sorted(tasks.size());
-        for (size_t q = 0; q < order.size(); ++q) sorted[q] = tasks[order[q]];
-        tasks.swap(sorted);
-    } else if (T == 4) {
-        std::stable_partition(tasks.begin(), tasks.end(), [seg](const int4& t) { return 4 * (t.z - t.y) >= seg; });
-    } else {
-        std::stable_sort(tasks.begin(), tasks.end(),
-                         [](const int4& x, const int4& y) { return x.z - x.y > y.z - y.y; });
-    }
+    const PlanBounds cap = plan_bounds(rule, nb, nt, nnz);
+    const size_t longs_at = sizeof(int4) * (size_t)cap.tasks, slots_at = longs_at + sizeof(int4) * (size_t)cap.longs;
     SpmmRowsPlan p;
     p.groups = T / (T <= 8 ? T : ROWS_R<32>);
-    p.ntasks = (int)tasks.size();
-    p.nlong = (int)longs.size();
-    p.nslots = nslots;
-    std::vector<int> slot_long((size_t)std::max(nslots, 1), 0);
-    for (int i = 0; i < p.nlong; ++i)
-        for (int q = 0; q < longs[i].z; ++q) slot_long[(size_t)longs[i].y + q] = i;
-    p.d_tasks = static_cast<int4*>(dev_alloc(sizeof(int4) * (size_t)std::max(p.ntasks, 1)));
-    p.d_long = static_cast<int4*>(dev_alloc(sizeof(int4) * (size_t)std::max(p.nlong, 1)));
-    p.d_slot_long = static_cast<int*>(dev_alloc(sizeof(int) * slot_long.size()));
-    if (!p.d_tasks || !p.d_long || !p.d_slot_long) {
-        spmm_rows_plan_free(&p);
-        return B2SR_ERR_ALLOC;
+    p.d_tasks = static_cast<int4*>(dev_alloc(slots_at + sizeof(int) * (size_t)cap.slots));
+    b2sr_status st = B2SR_ERR_ALLOC;
+    PlanTotals t;
+    if (p.d_tasks) {
+        p.d_long = p.d_tasks + cap.tasks;
+        p.d_slot_long = reinterpret_cast<int*>(p.d_long + cap.longs);
+        st = build_plan(rule, d_rowptr, nb, cap, p.d_tasks, p.d_long, p.d_slot_long, &t, s);
+    } else {
+        cudaStreamSynchronize(s);  // the set-bit count
     }
-    e = cudaSuccess;
-    if (p.ntasks) e = cudaMemcpy(p.d_tasks, tasks.data(), sizeof(int4) * (size_t)p.ntasks, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess && p.nlong)
-        e = cudaMemcpy(p.d_long, longs.data(), sizeof(int4) * (size_t)p.nlong, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess)
-        e = cudaMemcpy(p.d_slot_long, slot_long.data(), sizeof(int) * slot_long.size(), cudaMemcpyHostToDevice);
-    if (e != cudaSuccess) {
-        set_cuda_error(e);
+    dev_free(d_bits);
+    if (st != B2SR_SUCCESS) {
         spmm_rows_plan_free(&p);
-        return B2SR_ERR_CUDA;
+        return st;
     }
+    p.ntasks = t.tasks;
+    p.nlong = t.longs;
+    p.nslots = t.slots;
     *out = p;
     return B2SR_SUCCESS;
 }
 
 void spmm_rows_plan_free(SpmmRowsPlan* p) {
-    dev_free(p->d_tasks);
-    dev_free(p->d_long);
-    dev_free(p->d_slot_long);
+    dev_free(p->d_tasks);  // the others are part of it
     p->d_tasks = nullptr;
     p->d_long = nullptr;
     p->d_slot_long = nullptr;
