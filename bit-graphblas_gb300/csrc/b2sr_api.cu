@@ -48,8 +48,8 @@ static void* g_alloc_ctx = nullptr;
 
 // ---- device memory ---------------------------------------------------------------
 // Without a caller's allocator, device memory comes from one memory pool per
-// device that keeps up to 1/256 of the device's memory (1.1 GB on GB300) when it
-// is freed; more goes back to the driver at the next synchronization, and all of
+// device that keeps up to 1/256 of the device's memory (1.1 GB on GB300) beyond
+// what is in use when it is freed; more goes back to the driver at the next synchronization, and all of
 // it on b2sr_trim and before an allocation fails.  cudaMalloc takes 40 - 80 us
 // and cudaFree 30 - 110 us on GB300; packing a graph, transposing it and
 // building its plans makes some 50 such calls.
@@ -63,11 +63,23 @@ struct DevPool {
     cudaMemPool_t pool = nullptr;
     cudaStream_t stream = nullptr;
     bool tried = false;
+    uint64_t keep = 0, live = 0;  // bytes to keep beyond those in use; bytes in use
+};
+struct PoolBlock {
+    DevPool* pool;
+    size_t bytes;
 };
 constexpr int MAX_POOLS = 64;
 std::mutex g_pool_mu;
 DevPool g_pools[MAX_POOLS];
-std::unordered_map<void*, DevPool*> g_pool_blocks;  // live blocks of the pools
+std::unordered_map<void*, PoolBlock> g_pool_blocks;  // live blocks of the pools
+
+// The pool's threshold counts the bytes in use too.  With g_pool_mu held.
+cudaError_t pool_use(DevPool* p, uint64_t live) {
+    p->live = live;
+    uint64_t threshold = live + p->keep;
+    return cudaMemPoolSetAttribute(p->pool, cudaMemPoolAttrReleaseThreshold, &threshold);
+}
 
 // The device's pool, made on first use; null without one (then cudaMalloc).
 DevPool* device_pool(int dev) {
@@ -88,8 +100,8 @@ DevPool* device_pool(int dev) {
                   cudaStreamCreateWithFlags(&p.stream, cudaStreamNonBlocking) == cudaSuccess &&
                   cudaMemPoolCreate(&p.pool, &props) == cudaSuccess;
         if (ok) {
-            uint64_t keep = prop.totalGlobalMem / 256;
-            ok = cudaMemPoolSetAttribute(p.pool, cudaMemPoolAttrReleaseThreshold, &keep) == cudaSuccess;
+            p.keep = prop.totalGlobalMem / 256;
+            ok = pool_use(&p, 0) == cudaSuccess;
         }
         if (!ok) {
             if (p.pool) cudaMemPoolDestroy(p.pool);
@@ -132,7 +144,8 @@ void* dev_alloc(size_t bytes) {
         e = pool ? pool_alloc(pool, &p, bytes) : cudaMalloc(&p, bytes);
         if (pool && e == cudaSuccess) {
             std::lock_guard<std::mutex> lk(g_pool_mu);
-            g_pool_blocks[p] = pool;
+            g_pool_blocks[p] = {pool, bytes};
+            pool_use(pool, pool->live + bytes);
         }
     }
     if (e != cudaSuccess) {
@@ -162,7 +175,8 @@ void dev_free(void* p) {
         std::lock_guard<std::mutex> lk(g_pool_mu);
         auto it = g_pool_blocks.find(p);
         if (it != g_pool_blocks.end()) {
-            pool = it->second;
+            pool = it->second.pool;
+            pool_use(pool, pool->live - it->second.bytes);
             g_pool_blocks.erase(it);
         }
     }

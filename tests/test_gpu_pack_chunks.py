@@ -71,3 +71,30 @@ def test_batch_into_an_unaligned_array(pkg, orc, cuda, T):
     np.testing.assert_array_equal(bci.cpu().numpy(), wci)
     np.testing.assert_array_equal(got[1:-1], wtiles)
     assert got[0] == 5 and got[-1] == 5
+
+
+@pytest.mark.parametrize("T", [4, 8, 16, 32])
+def test_transpose_digit_passes(pkg, orc, cuda, T):
+    """One, two and three digit passes of the transpose's sort, with hub tile-columns; and wrapped tiles at an odd
+    byte address, with bits set in the unused half of a T = 4 row."""
+    rng = np.random.default_rng(T)
+    for ncols in (400 * T, 200000 * T, 300000 * T):
+        n, m = 600, 30000
+        rows, cols = rng.integers(0, n, m), rng.integers(0, ncols, m)
+        cols[: m // 3] = rng.integers(0, 5 * T, m // 3)
+        g = pkg.from_edges(rows, cols, nrows=n, ncols=ncols, drop_self_loops=False)
+        gt = pkg.from_edges(g.colind, np.repeat(np.arange(n), np.diff(g.rowptr)), nrows=ncols, ncols=n,
+                            drop_self_loops=False)
+        want = orc.csr_to_b2sr(gt.rowptr, gt.colind, ncols, T)
+        A = pkg.B2SRMatrix.from_graph(g, T, device=cuda)
+        for a, b in zip(A.transpose().download(), want):
+            np.testing.assert_array_equal(a, b)
+        rp, ci, tl = A.download()
+        A.close()
+        dirty = tl | 0x50 if T == 4 else tl
+        buf = torch.zeros(dirty.size + 1, dtype=pkg.word_dtype(T), device=cuda)
+        buf[1:] = torch.from_numpy(dirty.view(buf.cpu().numpy().dtype)).to(cuda)
+        B = pkg.B2SRMatrix.wrap(torch.from_numpy(rp).to(cuda), torch.from_numpy(ci).to(cuda), buf[1:], n, ncols, T)
+        for a, b in zip(B.transpose().download(), want):
+            np.testing.assert_array_equal(a, b)
+        B.close()
