@@ -1,23 +1,24 @@
 // Row-task B2SR x dense multiply: Y = A . X with X [ncols, k] and Y [nb*T, k]
 // row-major, FP32 or FP64 (bin_full_full on feature blocks; the adjoint
-// dX = A^T . dY is the same kernel on the transposed B2SR).  A task covers a
-// whole tile-row at T = 4 and 8, and one group of 8 of its rows at T = 16
-// and 32.
+// dX = A^T . dY is the same kernel on the transposed B2SR).  A work item is one
+// group of 4 rows of a task, T/4 items per task and column block.
 //
-// Plan (once per matrix, b2sr_plan.cu): one task per tile-row; a tile-row longer
-// than spmm_rows_seg() tiles (a share of one resident warp's part of all the
-// tiles) is cut into near-equal segments whose partial rows go to slots.  The warp that finishes a row's last segment (a per-row
-// arrival counter) adds the row's slots in segment order and writes Y, so a
-// multiply is one launch.  Warps take (column block, task) work items from a
-// device queue (an atomic counter); long tasks are handed out first, so the
-// queue ends on short ones (R-MAT hubs sit all over the vertex range, and in
-// row order the last items could be the longest).  The queue and
-// arrival counters live in a zeroed per-(matrix, stream) state buffer that
-// the kernel's last warp leaves zeroed again, so no launch needs a memset.
+// Plan (once per matrix, b2sr_plan.cu): one task per tile-row; a tile-row
+// longer than spmm_rows_seg() tiles (a share of one resident warp's part of all
+// the tiles), or at T >= 8 with more than such a share of the set bits, is cut
+// into near-equal segments whose partial rows go to slots.  The warp that
+// finishes a row's last segment (a per-row arrival counter) adds the row's
+// slots in segment order and writes Y, so a multiply is one launch.  Warps take
+// (column block, task, row group) work items from a device queue (an atomic
+// counter); long tasks are handed out first, so the queue ends on short ones
+// (R-MAT hubs sit all over the vertex range, and in row order the last items
+// could be the longest).  The queue and arrival counters live in a zeroed
+// per-(matrix, stream) state buffer that the kernel's last warp leaves zeroed
+// again, so no launch needs a memset.
 //
 // Inside a task a warp walks its tiles 32 at a time, one tile per lane.  The
-// lanes' set bits are appended to T item lists in shared memory, one per
-// tile row r, in tile then column order: the positions come from one warp
+// lanes' set bits are appended to 4 item lists in shared memory, one per row r
+// of the group, in tile then column order: the positions come from one warp
 // scan of the per-row bit counts (packed several rows to a word).  The lists
 // grow over many 32-tile steps (an R-MAT step holds ~8 items per row) and are
 // consumed only when one would overflow or the task ends, so a row's items
@@ -36,9 +37,7 @@ namespace b2sr {
 
 namespace {
 
-constexpr int ROWS_CAP = 256;    // item capacity of each tile row's region (ints); a step adds <= 32*T
 constexpr int ROWS_WARPS = 8;    // warps per block
-constexpr int ROWS_BATCH = 8;    // X-row loads in flight per lane
 
 template <typename V, int VEC> struct RowsVec;
 template <> struct RowsVec<float, 1> { using type = float; };
@@ -47,9 +46,13 @@ template <> struct RowsVec<float, 4> { using type = float4; };
 template <> struct RowsVec<double, 1> { using type = double; };
 template <> struct RowsVec<double, 2> { using type = double2; };
 
-template <typename V, int VEC>
-__device__ __forceinline__ void rows_load(V (&out)[VEC], const V* p, bool full, int nvalid) {
-    if (full) {
+// A lane's VEC columns of an X or Y row.  FULL: neighbouring columns, one
+// vector load (all VEC valid and aligned).  Otherwise columns STR apart (STR
+// lanes share the row), a coalesced scalar load each, the first nvalid of them
+// inside the row: widths and strides that are no multiple of 16 bytes.
+template <typename V, int VEC, bool FULL, int STR>
+__device__ __forceinline__ void rows_load(V (&out)[VEC], const V* p, int nvalid) {
+    if constexpr (FULL) {
         using VT = typename RowsVec<V, VEC>::type;
         const VT v = __ldg(reinterpret_cast<const VT*>(p));
         const V* e = reinterpret_cast<const V*>(&v);
@@ -57,7 +60,7 @@ __device__ __forceinline__ void rows_load(V (&out)[VEC], const V* p, bool full, 
         for (int i = 0; i < VEC; ++i) out[i] = e[i];
     } else {
 #pragma unroll
-        for (int i = 0; i < VEC; ++i) out[i] = i < nvalid ? __ldg(p + i) : V(0);
+        for (int i = 0; i < VEC; ++i) out[i] = i < nvalid ? __ldg(p + i * STR) : V(0);
     }
 }
 
@@ -74,16 +77,33 @@ __device__ __forceinline__ void rows_add(V (&acc)[VEC], const V (&v)[VEC]) {
             asm("add.rn.f32x2 %0, %0, %1;" : "+l"(x) : "l"(y));
             asm("mov.b64 {%0, %1}, %2;" : "=f"(acc[i]), "=f"(acc[i + 1]) : "l"(x));
         }
-        return;
-    }
+    } else {
 #pragma unroll
-    for (int e = 0; e < VEC; ++e) acc[e] += v[e];
+        for (int e = 0; e < VEC; ++e) acc[e] += v[e];
+    }
+}
+
+// acc += the N loaded rows: one after the other (FULL), or pairwise among
+// themselves first (the scalar layouts, which have one X row per load where
+// the vector ones have two partial sums per row at the same width).
+template <bool FULL, int N, typename V, int VEC>
+__device__ __forceinline__ void rows_add_all(V (&acc)[VEC], V (&v)[N][VEC]) {
+    if constexpr (!FULL) {
+#pragma unroll
+        for (int o = 1; o < N; o <<= 1)
+#pragma unroll
+            for (int u = 0; u < N; u += 2 * o) rows_add<V, VEC>(v[u], v[u + o]);
+        rows_add<V, VEC>(acc, v[0]);
+    } else {
+#pragma unroll
+        for (int u = 0; u < N; ++u) rows_add<V, VEC>(acc, v[u]);
+    }
 }
 
 // rows_load through L2 only (data written by other SMs in this launch)
-template <typename V, int VEC>
-__device__ __forceinline__ void rows_load_l2(V (&out)[VEC], const V* p, bool full, int nvalid) {
-    if (full) {
+template <typename V, int VEC, bool FULL, int STR>
+__device__ __forceinline__ void rows_load_l2(V (&out)[VEC], const V* p, int nvalid) {
+    if constexpr (FULL) {
         using VT = typename RowsVec<V, VEC>::type;
         const VT v = __ldcg(reinterpret_cast<const VT*>(p));
         const V* e = reinterpret_cast<const V*>(&v);
@@ -91,13 +111,13 @@ __device__ __forceinline__ void rows_load_l2(V (&out)[VEC], const V* p, bool ful
         for (int i = 0; i < VEC; ++i) out[i] = e[i];
     } else {
 #pragma unroll
-        for (int i = 0; i < VEC; ++i) out[i] = i < nvalid ? __ldcg(p + i) : V(0);
+        for (int i = 0; i < VEC; ++i) out[i] = i < nvalid ? __ldcg(p + i * STR) : V(0);
     }
 }
 
-template <typename V, int VEC>
-__device__ __forceinline__ void rows_store(V* p, const V (&v)[VEC], bool full, int nvalid, bool accumulate) {
-    if (full) {
+template <typename V, int VEC, bool FULL, int STR>
+__device__ __forceinline__ void rows_store(V* p, const V (&v)[VEC], int nvalid, bool accumulate) {
+    if constexpr (FULL) {
         using VT = typename RowsVec<V, VEC>::type;
         VT* q = reinterpret_cast<VT*>(p);
         VT o;
@@ -115,68 +135,62 @@ __device__ __forceinline__ void rows_store(V* p, const V (&v)[VEC], bool full, i
     } else {
 #pragma unroll
         for (int i = 0; i < VEC; ++i)
-            if (i < nvalid) p[i] = accumulate ? p[i] + v[i] : v[i];
+            if (i < nvalid) p[i * STR] = accumulate ? p[i * STR] + v[i] : v[i];
     }
 }
 
-// Rows of a tile-row one task covers: all of them at T = 4 and 8; at T = 16
-// and 32 a task is one group of 8 rows (G = T / 8 groups per tile-row, each
-// its own work item), so its accumulators, item lists and occupancy are those
-// of T = 8.  Groups of 8 rows walk each tile half as often as groups of 4:
-// R-MAT scale 18, k = 64: 0.496 / 1.041 ms at T = 16 / 32 against 0.600 /
-// 1.283 ms with groups of 4 (the merge-path kernel: 3.00 / 14.7 ms).
-template <int T> constexpr int ROWS_R = T <= 8 ? T : 8;
-// blocks of ROWS_WARPS warps per SM the register budget is written for
-template <int T> constexpr int ROWS_BLOCKS = ROWS_R<T> == 4 ? 4 : 2;
+// Rows of a tile-row one task covers: 4, so G = T/4 work items per tile-row.
+// A task's accumulators (4 rows x 16 bytes of columns a lane) and loads in
+// flight then fit 64 registers at every T, four blocks per SM, and an item's
+// rows are few enough for long runs.  With 8 rows (whole tile-rows at T = 8,
+// two blocks per SM) each tile was read half as often, but short rows left
+// the loads of 16 warps waiting: R-MAT scale 18, k = 64 / 128: T = 8 228 / 407
+// -> 197 / 291 us, T = 16 292 / 484 -> 265 / 350 us, T = 32 372 / 544 -> 361 /
+// 449 us; 100,003-vertex ER graph of degree 11, k = 50: T = 8 64 -> 46 us,
+// T = 32 146 -> 107 us.
+constexpr int ROWS_R = 4;
+constexpr int ROWS_BLOCKS = 4;   // blocks of ROWS_WARPS warps per SM the register budget is written for
+constexpr int ROWS_CAP = 256;    // item capacity of each tile row's region in shared memory; a step adds <= 32*T
+constexpr int ROWS_BATCH = 8;    // X-row loads in flight per lane
+constexpr int ROWS_REST = 4;     // and of the rest of a list
 
 // Packed per-row bit counts: FIELD bits per row (a row total over 32 lanes
 // is at most 32*T: 128 fits 8 bits for T = 4; 256, 512 and 1024 take 16).
 template <int T> struct RowsPack {
     static constexpr int FIELD = T == 4 ? 8 : 16;
     static constexpr int PER = 32 / FIELD;        // rows per 32-bit pack
-    static constexpr int NP = ROWS_R<T> / PER;    // packs
+    static constexpr int NP = ROWS_R / PER;    // packs
     static constexpr uint32_t MASK = (1u << FIELD) - 1;
 };
 
-// The rows of lane's tile that its task covers.  T = 4 / 8: the whole tile as
-// 64 bits, row r in byte r (T = 4: low nibble).  T = 16 / 32: rows
-// R*g .. R*g+R-1 of group g, R*T/32 words read with 16-byte loads.
-// bits(r): row r's word, bit T-1-c = column c.
-template <int T> struct RowsWordNarrow {
-    unsigned long long w = 0;
-    __device__ __forceinline__ void load(const void* tiles, int j, int) {
-        if constexpr (T == 4) {
-            w = __ldg(static_cast<const unsigned int*>(tiles) + j);
-        } else {
-            const uint2 v = __ldg(static_cast<const uint2*>(tiles) + j);
-            w = ((unsigned long long)v.y << 32) | v.x;
-        }
-    }
-    __device__ __forceinline__ uint32_t bits(int r) const { return (uint32_t)(w >> (8 * r)) & ((1u << T) - 1u); }
-};
-template <int T> struct RowsWordWide {
-    static constexpr int NW = ROWS_R<T> * T / 32;  // 32-bit words of a group: 4 (T = 16), 8 (T = 32)
-    static_assert(NW % 4 == 0, "a group is whole 16-byte words");
+// The rows of lane's tile that its task covers: rows 4*g .. 4*g+3 of group g,
+// T/8 words read with one load.  bits(r): row r's word, bit T-1-c = column c.
+template <int T> struct RowsWord {
+    static constexpr int NW = T <= 8 ? 1 : T / 8;
     uint32_t w[NW] = {};
     __device__ __forceinline__ void load(const void* tiles, int j, int g) {
-        // byte offset j*T*T/8 + g*NW*4: a multiple of 16
-        const uint32_t* p = static_cast<const uint32_t*>(tiles) + (size_t)j * (T * T / 32) + (size_t)g * NW;
-#pragma unroll
-        for (int i = 0; i < NW / 4; ++i) {
-            const uint4 v = __ldg(reinterpret_cast<const uint4*>(p) + i);
-            w[4 * i] = v.x;
-            w[4 * i + 1] = v.y;
-            w[4 * i + 2] = v.z;
-            w[4 * i + 3] = v.w;
+        // byte offset (j*T/4 + g) * NW*4: a multiple of the load's size
+        const size_t at = (size_t)j * (T / ROWS_R) + g;
+        if constexpr (NW == 4) {
+            const uint4 v = __ldg(static_cast<const uint4*>(tiles) + at);
+            w[0] = v.x;
+            w[1] = v.y;
+            w[2] = v.z;
+            w[3] = v.w;
+        } else if constexpr (NW == 2) {
+            const uint2 v = __ldg(static_cast<const uint2*>(tiles) + at);
+            w[0] = v.x;
+            w[1] = v.y;
+        } else {
+            w[0] = __ldg(static_cast<const uint32_t*>(tiles) + at);
         }
     }
     __device__ __forceinline__ uint32_t bits(int r) const {
-        if constexpr (T == 16) return (w[r >> 1] >> (16 * (r & 1))) & 0xffffu;
-        else return w[r];
+        if constexpr (T == 32) return w[r];
+        else if constexpr (T == 16) return (w[r >> 1] >> (16 * (r & 1))) & 0xffffu;
+        else return (w[0] >> (8 * r)) & ((1u << T) - 1u);
     }
 };
-template <int T>
-using RowsWord = typename std::conditional<(T <= 8), RowsWordNarrow<T>, RowsWordWide<T>>::type;
 
 }  // namespace
 
@@ -202,24 +216,28 @@ struct SpmmRowsArgs {
 // r0 .. r0+R-1 of its tile-row): those Y rows (+)= the row's slots added in
 // segment order, over all k columns (every column block of the group has
 // arrived); sub-group `sub` takes rows r0+sub, r0+sub+IPW, ...  SL slots in
-// flight (2 with whole tile-rows, whose main loop needs the registers; 8 with
-// 8-row groups at T = 16 / 32, whose long rows have the most slots), added
-// in slot order; no unrolling of the outer loops (an out-of-line call
+// flight (the main loop needs the registers), added in slot order; no unrolling of the outer loops (an out-of-line call
 // measured slower).
-template <int T, int IPW, bool FULL, typename V>
+// First column of a lane in column block cb, and how many columns it has there.
+template <int VEC, int LPI, bool FULL>
+__device__ __forceinline__ int rows_col(int cb, int lane, int k, int& nvalid) {
+    const int col = cb * LPI * VEC + (lane % LPI) * (FULL ? VEC : 1);
+    nvalid = FULL ? max(0, min(VEC, k - col)) : max(0, min(VEC, (k - col + LPI - 1) / LPI));
+    return col;
+}
+
+template <int T, int IPW, int VEC, bool FULL, typename V>
 __device__ __forceinline__ void rows_long_reduce(const SpmmRowsArgs<V>& a, int lr, int lane, int r0) {
-    constexpr int VEC = 16 / (int)sizeof(V);
     constexpr int LPI = 32 / IPW;
-    constexpr int KC = LPI * VEC;
-    constexpr int R = ROWS_R<T>;
-    constexpr int SL = T >= 16 ? 8 : 2;
+    constexpr int R = ROWS_R;
+    constexpr int SL = 2;
     const int sub = lane / LPI;
     const int4 L = __ldg(a.long_rows + lr);
     const long long stride = (long long)T * a.k;
 #pragma unroll 1
     for (int cb = 0; cb < a.ncb; ++cb) {
-        const int col = cb * KC + (lane % LPI) * VEC;
-        const int nvalid = max(0, min(VEC, a.k - col));
+        int nvalid;
+        const int col = rows_col<VEC, LPI, FULL>(cb, lane, a.k, nvalid);
         if (nvalid == 0) continue;
 #pragma unroll 1
         for (int r = r0 + sub; r < r0 + R; r += IPW) {
@@ -232,7 +250,7 @@ __device__ __forceinline__ void rows_long_reduce(const SpmmRowsArgs<V>& a, int l
             for (; q + SL - 1 < L.z; q += SL) {
                 V v[SL][VEC];
 #pragma unroll
-                for (int u = 0; u < SL; ++u) rows_load_l2<V, VEC>(v[u], src + (q + u) * stride, FULL, nvalid);
+                for (int u = 0; u < SL; ++u) rows_load_l2<V, VEC, FULL, LPI>(v[u], src + (q + u) * stride, nvalid);
 #pragma unroll
                 for (int u = 0; u < SL; ++u)
 #pragma unroll
@@ -241,35 +259,34 @@ __device__ __forceinline__ void rows_long_reduce(const SpmmRowsArgs<V>& a, int l
 #pragma unroll 1
             for (; q < L.z; ++q) {
                 V v0[VEC];
-                rows_load_l2<V, VEC>(v0, src + q * stride, FULL, nvalid);
+                rows_load_l2<V, VEC, FULL, LPI>(v0, src + q * stride, nvalid);
 #pragma unroll
                 for (int e = 0; e < VEC; ++e) tot[e] += v0[e];
             }
-            rows_store<V, VEC>(a.Y + ((long long)L.x * T + r) * a.ldy + col, tot, FULL, nvalid,
-                               a.accumulate != 0);
+            rows_store<V, VEC, FULL, LPI>(a.Y + ((long long)L.x * T + r) * a.ldy + col, tot, nvalid,
+                                          a.accumulate != 0);
         }
     }
 }
 
-// VEC = 16 bytes of columns per lane; a warp loads IPW items (X rows) per
-// instruction, LPI = 32/IPW lanes per item, so a column block is LPI*VEC
-// columns (k = 64 FP32: two X rows per warp load).  FULL: every column
-// vector is whole and 16-byte aligned (else per-element guarded loads).
+// A lane holds VEC columns, LPI = 32/IPW lanes a column block of LPI*VEC
+// columns, and a warp loads IPW items (X rows) per instruction (k = 64 FP32:
+// two X rows of 16 lanes x 16 bytes).  FULL: 16 bytes of neighbouring columns
+// per lane, every vector whole and aligned.  Otherwise rows_width() picks as
+// few scalar columns per lane as cover k.
 // Work item wi = (column block, task, row group), the group fastest, so the
 // G warps of one tile-row read its structure at about the same time.
-template <int T, int IPW, bool FULL, typename V>
-__global__ void __launch_bounds__(ROWS_WARPS * 32, ROWS_BLOCKS<T>)
+template <int T, int IPW, int VEC, bool FULL, typename V>
+__global__ void __launch_bounds__(ROWS_WARPS * 32, ROWS_BLOCKS)
 spmm_rows_kernel(SpmmRowsArgs<V> a) {
     using P = RowsPack<T>;
-    constexpr int R = ROWS_R<T>;  // rows per task
+    constexpr int R = ROWS_R;  // rows per task
     constexpr int G = T / R;      // row groups per tile-row
     // a step of 32 tiles adds at most 32*T items to a row: more than a region
     // holds only at T >= 16, where such a step is appended in lane ranges
     constexpr bool SPLIT = 32 * T > ROWS_CAP;
     static_assert(T <= ROWS_CAP, "one tile's items of a row must fit an empty region");
-    constexpr int VEC = 16 / (int)sizeof(V);
     constexpr int LPI = 32 / IPW;
-    constexpr int KC = LPI * VEC;
     extern __shared__ int s_items[];  // per warp: R regions of ROWS_CAP items
     const int lane = threadIdx.x & 31;
     const int sub = lane / LPI;  // which item of an instruction this lane loads
@@ -277,8 +294,8 @@ spmm_rows_kernel(SpmmRowsArgs<V> a) {
     const long long nwork = (long long)a.ntasks * a.ncb * G;
     const unsigned ldx = (unsigned)a.ldx;
     while (true) {
-        int wi = 0;
-        if (lane == 0) wi = atomicAdd(a.state, 1);
+        unsigned wi = 0;
+        if (lane == 0) wi = atomicAdd(reinterpret_cast<unsigned*>(a.state), 1u);
         wi = __shfl_sync(FULL_MASK, wi, 0);
         if (wi >= nwork) {
             // every warp fetches past the end exactly once; the last one to
@@ -293,12 +310,12 @@ spmm_rows_kernel(SpmmRowsArgs<V> a) {
             break;
         }
         // column block major: one pass over the tasks per block of X columns
-        const int gi = G == 1 ? 0 : wi % G;
-        const int wt = G == 1 ? wi : wi / G;
-        const int cb = wt / a.ntasks, task = wt - cb * a.ntasks;
+        const int gi = (int)(wi % G);
+        const unsigned wt = wi / G;
+        const int cb = (int)(wt / (unsigned)a.ntasks), task = (int)(wt - (unsigned)cb * (unsigned)a.ntasks);
         const int4 t = __ldg(a.tasks + task);
-        const int col = cb * KC + (lane % LPI) * VEC;
-        const int nvalid = max(0, min(VEC, a.k - col));
+        int nvalid;
+        const int col = rows_col<VEC, LPI, FULL>(cb, lane, a.k, nvalid);
         const bool active = nvalid > 0;
         const V* xc = a.X + col;
         V acc[R][VEC];
@@ -391,25 +408,23 @@ spmm_rows_kernel(SpmmRowsArgs<V> a) {
 #pragma unroll
                                 for (int u = 0; u < ROWS_BATCH; ++u) {
                                     const unsigned xr = (unsigned)it[q + u * IPW];
-                                    rows_load<V, VEC>(xv[u], xc + (size_t)xr * ldx, FULL, nvalid);
+                                    rows_load<V, VEC, FULL, LPI>(xv[u], xc + (size_t)xr * ldx, nvalid);
                                 }
-#pragma unroll
-                                for (int u = 0; u < ROWS_BATCH; ++u) rows_add<V, VEC>(acc[r], xv[u]);
+                                rows_add_all<FULL, ROWS_BATCH, V, VEC>(acc[r], xv);
                             }
-                            for (; q < qb; q += 4 * IPW) {  // the rest, four loads per lane per round
-                                V xv[4][VEC];
+                            for (; q < qb; q += ROWS_REST * IPW) {  // the rest, ROWS_REST loads per lane per round
+                                V xv[ROWS_REST][VEC];
 #pragma unroll
-                                for (int u = 0; u < 4; ++u) {
+                                for (int u = 0; u < ROWS_REST; ++u) {
                                     if (q + u * IPW < qb) {
-                                        rows_load<V, VEC>(xv[u], xc + (size_t)(unsigned)it[q + u * IPW] * ldx, FULL,
-                                                          nvalid);
+                                        rows_load<V, VEC, FULL, LPI>(
+                                            xv[u], xc + (size_t)(unsigned)it[q + u * IPW] * ldx, nvalid);
                                     } else {
 #pragma unroll
                                         for (int e = 0; e < VEC; ++e) xv[u][e] = V(0);
                                     }
                                 }
-#pragma unroll
-                                for (int u = 0; u < 4; ++u) rows_add<V, VEC>(acc[r], xv[u]);
+                                rows_add_all<FULL, ROWS_REST, V, VEC>(acc[r], xv);
                             }
                         }
                     }
@@ -453,8 +468,8 @@ spmm_rows_kernel(SpmmRowsArgs<V> a) {
             if (writer) {
 #pragma unroll
                 for (int r = 0; r < R; ++r)
-                    rows_store<V, VEC>(a.Y + ((long long)t.x * T + r0 + r) * a.ldy + col, acc[r], FULL, nvalid,
-                                       a.accumulate != 0);
+                    rows_store<V, VEC, FULL, LPI>(a.Y + ((long long)t.x * T + r0 + r) * a.ldy + col, acc[r], nvalid,
+                                                  a.accumulate != 0);
             }
             continue;
         }
@@ -462,7 +477,7 @@ spmm_rows_kernel(SpmmRowsArgs<V> a) {
         V* dst = a.partials + ((long long)t.w * T + r0) * a.k + col;
         if (writer) {
 #pragma unroll
-            for (int r = 0; r < R; ++r) rows_store<V, VEC>(dst + (long long)r * a.k, acc[r], FULL, nvalid, false);
+            for (int r = 0; r < R; ++r) rows_store<V, VEC, FULL, LPI>(dst + (long long)r * a.k, acc[r], nvalid, false);
         }
         __threadfence();
         __syncwarp();
@@ -476,25 +491,21 @@ spmm_rows_kernel(SpmmRowsArgs<V> a) {
         // the group's last segment: its Y rows (+)= its slots added in segment order
         lr = __shfl_sync(FULL_MASK, lr, 0);
         __threadfence();
-        rows_long_reduce<T, IPW, FULL, V>(a, lr, lane, r0);
+        rows_long_reduce<T, IPW, VEC, FULL, V>(a, lr, lane, r0);
         if (lane == 0) a.state[2 + lr * G + gi] = 0;
     }
 }
 
 // ---- plan ---------------------------------------------------------------------------
-// Longest task in tiles: a fixed share of one resident warp's part of the
-// tile visits (4 blocks of 8 warps per SM with 4-row tasks, 2 with 8-row
-// tasks), so that the queue stays balanced at every graph size.  The shares,
-// 30% with 4-row tasks and 20% with 8-row tasks, were the best of 20/30/40%
-// on R-MAT scales 16-20 with k = 64 and 128 on GB300; 40% fell off a cliff
-// (the queue's end waits on long segments).  At T = 16 / 32 a task's tiles
-// are walked once per row group, so the visits are nt x T/8.
+// Longest task in tiles: 30% of one resident warp's part of the tile visits
+// (nt x T/4: a task's tiles are walked once per row group), so that the queue
+// stays balanced at every graph size.  The best of 20/30/40% on R-MAT scales
+// 16-20 with k = 64 and 128 on GB300; 40% fell off a cliff at T = 4 (the
+// queue's end waits on long segments).
 int spmm_rows_seg(int T, long long nt, int num_sms) {
-    const int R = T <= 8 ? T : ROWS_R<32>;
-    const long long visits = nt * (T / R);
-    const long long warps = (long long)std::max(num_sms, 1) * (R == 4 ? 4 : 2) * ROWS_WARPS;
-    const long long pct = R == 4 ? 30 : 20;
-    return (int)std::min(8192LL, std::max(128LL, visits * pct / (100 * warps)));
+    const long long visits = nt * (T / ROWS_R);
+    const long long warps = (long long)std::max(num_sms, 1) * ROWS_BLOCKS * ROWS_WARPS;
+    return (int)std::min(8192LL, std::max(128LL, visits * 30 / (100 * warps)));
 }
 
 // Set bits of every tile-row: one warp per tile-row (grid-stride), popc of
@@ -520,34 +531,31 @@ b2sr_status spmm_rows_plan_create(const int* d_rowptr, const void* d_tiles, int 
     // tasks while tile-rows that share X rows (the blocks of a batched graph)
     // still run together: R-MAT scale 18 / 20 as fast as longest first, and
     // 512 stacked ER graphs 1.86 ms against 2.85 ms longest first (2.61 ms in
-    // row order with fixed segments).  T = 8: longest first (R-MAT scale 18:
-    // 0.233 against 0.268 ms with the split).  T = 16 / 32: most set bits
-    // first.
-    PlanRule rule{T == 4 ? PlanRule::TWO : T == 8 ? PlanRule::LENGTH : PlanRule::BITS, spmm_rows_seg(T, nt, num_sms),
-                  T == 4 ? 2 : PLAN_CLASSES};
-    // T = 16 / 32: the set bits of every tile-row.  A row group holding hub
-    // rows carries far more set bits than its tiles suggest (R-MAT scale 18,
-    // T = 32: ~9.3 K X-row loads for one warp in a tile-bounded segment of
-    // tile-row 0, against 3.1 K set bits per resident warp on average),
-    // so there segments are also bounded by set bits: at most one resident
-    // warp's average share of all the bits (with the queue ordered by set
-    // bits and the long rows reduced per row group: R-MAT scale 18, k = 64,
-    // 0.295 / 0.377 ms at T = 16 / 32 against 0.484 / 1.027 ms with
-    // tile-bounded segments).
+    // row order with fixed segments).
+    PlanRule rule{T == 4 ? PlanRule::TWO : PlanRule::BITS, spmm_rows_seg(T, nt, num_sms), T == 4 ? 2 : PLAN_CLASSES};
+    // T >= 8: segments also bounded by their set bits, at most 70% of a
+    // resident warp's share of all of them, and most set bits first.  A row
+    // group holding hub rows carries far more set bits than its tiles suggest
+    // (R-MAT scale 18, T = 32: ~9.3 K X-row loads for one warp in a
+    // tile-bounded segment of tile-row 0, against 3.1 K set bits per resident
+    // warp on average).  R-MAT scale 18, T = 8, k = 64 / 128: 198 / 291 us
+    // against 249 / 469 us longest first; 100% instead of 70%: T = 32, k = 128
+    // 535 instead of 449 us, 50%: T = 16, k = 33 298 instead of 269 us.
     long long* d_bits = nullptr;
-    if (T >= 16 && nb > 0) {
+    if (T >= 8 && nb > 0) {
         d_bits = static_cast<long long*>(dev_alloc(sizeof(long long) * (size_t)nb));
         if (!d_bits) return B2SR_ERR_ALLOC;
         const long long blocks = std::min<long long>(((long long)nb * 32 + 255) / 256, 65535LL * 8);
         tile_row_bits_kernel<<<(unsigned)blocks, 256, 0, s>>>(d_rowptr, static_cast<const uint32_t*>(d_tiles), nb,
                                                                 T * T / 32, d_bits);
         rule.row_bits = d_bits;
-        rule.seg_bits = std::max(1024LL, nnz / ((long long)std::max(num_sms, 1) * ROWS_BLOCKS<32> * ROWS_WARPS));
+        const long long warps = (long long)std::max(num_sms, 1) * ROWS_BLOCKS * ROWS_WARPS;
+        rule.seg_bits = std::max(1024LL, nnz * 7 / (10 * warps));
     }
     const PlanBounds cap = plan_bounds(rule, nb, nt, nnz);
     const size_t longs_at = sizeof(int4) * (size_t)cap.tasks, slots_at = longs_at + sizeof(int4) * (size_t)cap.longs;
     SpmmRowsPlan p;
-    p.groups = T / (T <= 8 ? T : ROWS_R<32>);
+    p.groups = T / ROWS_R;
     p.d_tasks = static_cast<int4*>(dev_alloc(slots_at + sizeof(int) * (size_t)cap.slots));
     b2sr_status st = B2SR_ERR_ALLOC;
     PlanTotals t;
@@ -577,20 +585,21 @@ void spmm_rows_plan_free(SpmmRowsPlan* p) {
     p->d_slot_long = nullptr;
 }
 
-// Items per warp load.  rhs_block > 0 (FP32 columns; half as many FP64
-// columns) fixes the column block 32/IPW lanes x 16 bytes; 0 takes the
-// largest power of two IPW (at most 8) whose block still covers k.
-static int rows_ipw(int elem_bytes, int k, int rhs_block) {
-    const int vec = 16 / elem_bytes;
-    if (rhs_block > 0) {
-        const int cols = rhs_block * 4 / elem_bytes;  // columns of this element size
-        int ipw = 1;
-        while (ipw < 8 && (32 / (2 * ipw)) * vec >= cols) ipw *= 2;
-        return ipw;
-    }
-    int ipw = 1;
-    while (ipw < 8 && (32 / (2 * ipw)) * vec >= k) ipw *= 2;
-    return ipw;
+// Columns of a warp pass (LPI * VEC) and of a lane.  rhs_block > 0 (FP32
+// columns; half as many FP64 columns) fixes the block; 0 takes the narrowest
+// that covers k.  Vector lanes (FULL): 16 bytes each, 4 to 32 lanes a row.
+// Scalar lanes: one column each up to 32 columns (IPW rows per load below
+// that), else 32 lanes of 2, 3 or 4 columns (FP64: 2).
+struct RowsWidth {
+    int ipw, vec;
+};
+static RowsWidth rows_width(int elem_bytes, int k, int rhs_block, bool full) {
+    const int cols = rhs_block > 0 ? rhs_block * 4 / elem_bytes : k;
+    RowsWidth w{1, full ? 16 / elem_bytes : 1};
+    while (w.ipw < 8 && (32 / (2 * w.ipw)) * w.vec >= cols) w.ipw *= 2;
+    const int most = 16 / elem_bytes;
+    while (!full && w.vec < most && 32 * w.vec < cols) ++w.vec;
+    return w;
 }
 
 size_t spmm_rows_scratch_bytes(const SpmmRowsPlan& p, int T, int elem_bytes, int k) {
@@ -599,11 +608,11 @@ size_t spmm_rows_scratch_bytes(const SpmmRowsPlan& p, int T, int elem_bytes, int
 
 size_t spmm_rows_state_bytes(const SpmmRowsPlan& p) { return sizeof(int) * (2 + (size_t)p.nlong * p.groups); }
 
-template <int T, int IPW, bool FULL, typename V>
-static b2sr_status run_rows(SpmmRowsArgs<V> a, const SpmmRowsPlan& p, int num_sms, cudaStream_t s) {
-    constexpr int SMEM = ROWS_WARPS * ROWS_R<T> * ROWS_CAP * (int)sizeof(int);
+template <int T, int IPW, int VEC, bool FULL, typename V>
+static b2sr_status run_rows(SpmmRowsArgs<V> a, int num_sms, cudaStream_t s) {
+    constexpr int SMEM = ROWS_WARPS * ROWS_R * ROWS_CAP * (int)sizeof(int);
     // per device: the attribute is set on every launch (cheap), the occupancy once
-    cudaError_t e = cudaFuncSetAttribute(spmm_rows_kernel<T, IPW, FULL, V>,
+    cudaError_t e = cudaFuncSetAttribute(spmm_rows_kernel<T, IPW, VEC, FULL, V>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
     if (e != cudaSuccess) {
         set_cuda_error(e);
@@ -612,7 +621,7 @@ static b2sr_status run_rows(SpmmRowsArgs<V> a, const SpmmRowsPlan& p, int num_sm
     static int blocks_per_sm = 0;  // per instantiation; the device's SM count scales it
     if (blocks_per_sm == 0) {
         int n = 0;
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, spmm_rows_kernel<T, IPW, FULL, V>, ROWS_WARPS * 32,
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, spmm_rows_kernel<T, IPW, VEC, FULL, V>, ROWS_WARPS * 32,
                                                           SMEM);
         if (e != cudaSuccess) {
             set_cuda_error(e);
@@ -620,14 +629,13 @@ static b2sr_status run_rows(SpmmRowsArgs<V> a, const SpmmRowsPlan& p, int num_sm
         }
         blocks_per_sm = std::max(n, 1);
     }
-    const long long nwork = (long long)a.ntasks * a.ncb * (T / ROWS_R<T>);
+    const long long nwork = (long long)a.ntasks * a.ncb * (T / ROWS_R);
     const long long want = (nwork + ROWS_WARPS - 1) / ROWS_WARPS;
     const int grid = (int)std::max(1LL, std::min<long long>((long long)num_sms * blocks_per_sm, want));
-    // the queue counter is a 32-bit int that ends at nwork + one fetch per
-    // warp, and a long row's arrivals count to its slots x ncb
-    if (nwork + (long long)grid * ROWS_WARPS >= 0x7fffffffLL) return B2SR_ERR_NOT_SUPPORTED;
+    // the queue counter is 32 bits and ends at nwork + one fetch per warp
+    if (nwork + (long long)grid * ROWS_WARPS >= 0xffffffffLL) return B2SR_ERR_NOT_SUPPORTED;
     kernel_timer_mark(s, true);
-    spmm_rows_kernel<T, IPW, FULL, V><<<grid, ROWS_WARPS * 32, SMEM, s>>>(a);
+    spmm_rows_kernel<T, IPW, VEC, FULL, V><<<grid, ROWS_WARPS * 32, SMEM, s>>>(a);
     kernel_timer_mark(s, false);
     B2SR_LAUNCH_CHECK();
     add_launch_count(1);
@@ -635,14 +643,27 @@ static b2sr_status run_rows(SpmmRowsArgs<V> a, const SpmmRowsPlan& p, int num_sm
 }
 
 template <int T, typename V>
-static b2sr_status rows_dispatch(const SpmmRowsArgs<V>& a, int ipw, bool full, const SpmmRowsPlan& p, int num_sms,
-                                 cudaStream_t s) {
-#define B2SR_ROWS_IPW(I)                                                   \
-    if (ipw == I) return full ? run_rows<T, I, true, V>(a, p, num_sms, s) \
-                              : run_rows<T, I, false, V>(a, p, num_sms, s);
-    B2SR_ROWS_IPW(1) B2SR_ROWS_IPW(2) B2SR_ROWS_IPW(4) B2SR_ROWS_IPW(8)
-#undef B2SR_ROWS_IPW
-    return B2SR_ERR_INVALID_VALUE;
+static b2sr_status rows_dispatch(const SpmmRowsArgs<V>& a, RowsWidth w, bool full, int num_sms, cudaStream_t s) {
+    constexpr int MOST = 16 / (int)sizeof(V);
+    if (full) {
+        switch (w.ipw) {
+            case 1: return run_rows<T, 1, MOST, true, V>(a, num_sms, s);
+            case 2: return run_rows<T, 2, MOST, true, V>(a, num_sms, s);
+            case 4: return run_rows<T, 4, MOST, true, V>(a, num_sms, s);
+            default: return run_rows<T, 8, MOST, true, V>(a, num_sms, s);
+        }
+    }
+    if (w.vec == 2) return run_rows<T, 1, 2, false, V>(a, num_sms, s);
+    if constexpr (MOST == 4) {
+        if (w.vec == 3) return run_rows<T, 1, 3, false, V>(a, num_sms, s);
+        if (w.vec == 4) return run_rows<T, 1, 4, false, V>(a, num_sms, s);
+    }
+    switch (w.ipw) {
+        case 1: return run_rows<T, 1, 1, false, V>(a, num_sms, s);
+        case 2: return run_rows<T, 2, 1, false, V>(a, num_sms, s);
+        case 4: return run_rows<T, 4, 1, false, V>(a, num_sms, s);
+        default: return run_rows<T, 8, 1, false, V>(a, num_sms, s);
+    }
 }
 
 template <typename V>
@@ -651,8 +672,11 @@ b2sr_status spmm_rows_launch(const MatView& A, const SpmmRowsPlan& p, const V* X
                              int num_sms, cudaStream_t s) {
     constexpr int VEC = 16 / (int)sizeof(V);
     if (ldx > 0x7fffffffLL) return B2SR_ERR_NOT_SUPPORTED;
-    const int ipw = rows_ipw((int)sizeof(V), k, rhs_block);
-    const int KC = (32 / ipw) * VEC;
+    // whole 16-byte column vectors everywhere: X, Y aligned, row strides and k multiples of VEC
+    const bool full = ((uintptr_t)X % 16 == 0) && ((uintptr_t)Y % 16 == 0) && (ldx % VEC == 0) &&
+                      (ldy % VEC == 0) && (k % VEC == 0);
+    const RowsWidth w = rows_width((int)sizeof(V), k, rhs_block, full);
+    const int KC = (32 / w.ipw) * w.vec;
     SpmmRowsArgs<V> a;
     a.colind = A.colind;
     a.tiles = A.tiles;
@@ -669,13 +693,10 @@ b2sr_status spmm_rows_launch(const MatView& A, const SpmmRowsPlan& p, const V* X
     a.slot_long = p.d_slot_long;
     a.partials = static_cast<V*>(scratch);
     a.accumulate = accumulate;
-    // whole 16-byte column vectors everywhere: X, Y aligned, row strides and k multiples of VEC
-    const bool full = ((uintptr_t)X % 16 == 0) && ((uintptr_t)Y % 16 == 0) && (ldx % VEC == 0) &&
-                      (ldy % VEC == 0) && (k % VEC == 0);
-    if (A.T == 4) return rows_dispatch<4, V>(a, ipw, full, p, num_sms, s);
-    if (A.T == 8) return rows_dispatch<8, V>(a, ipw, full, p, num_sms, s);
-    if (A.T == 16) return rows_dispatch<16, V>(a, ipw, full, p, num_sms, s);
-    if (A.T == 32) return rows_dispatch<32, V>(a, ipw, full, p, num_sms, s);
+    if (A.T == 4) return rows_dispatch<4, V>(a, w, full, num_sms, s);
+    if (A.T == 8) return rows_dispatch<8, V>(a, w, full, num_sms, s);
+    if (A.T == 16) return rows_dispatch<16, V>(a, w, full, num_sms, s);
+    if (A.T == 32) return rows_dispatch<32, V>(a, w, full, num_sms, s);
     return B2SR_ERR_INVALID_VALUE;
 }
 
