@@ -341,34 +341,25 @@ static int* matrix_auto_hint(b2sr_matrix* m) {
     return m->auto_hint;
 }
 
-// Side stream, events and zeroed count state of m for stream s (created once).
-static b2sr_status matrix_auto_side(b2sr_matrix* m, cudaStream_t s, b2sr_matrix::AutoSide** out) {
+// The auto direction's counters of m for stream s: [0..1] the push's, [2..3]
+// the count's beside a hinted pull; zeroed on s when created.
+static b2sr_status matrix_auto_state(b2sr_matrix* m, cudaStream_t s, int** out) {
     std::lock_guard<std::mutex> lk(m->scratch_mu);
-    for (auto& e : m->auto_side)
+    for (auto& e : m->auto_state)
         if (e.stream == s) {
-            *out = &e;
+            *out = static_cast<int*>(e.ptr);
             return B2SR_SUCCESS;
         }
-    b2sr_matrix::AutoSide e{s, nullptr, nullptr, nullptr, nullptr};
-    cudaError_t err = cudaStreamCreateWithFlags(&e.side, cudaStreamNonBlocking);
-    if (err == cudaSuccess) err = cudaEventCreateWithFlags(&e.fork, cudaEventDisableTiming);
-    if (err == cudaSuccess) err = cudaEventCreateWithFlags(&e.join, cudaEventDisableTiming);
-    if (err == cudaSuccess) {
-        e.state = static_cast<int*>(dev_alloc(4 * sizeof(int)));
-        if (!e.state) err = cudaErrorMemoryAllocation;
-    }
-    if (err == cudaSuccess) err = cudaMemsetAsync(e.state, 0, 4 * sizeof(int), e.side);
-    if (err == cudaSuccess) err = cudaStreamSynchronize(e.side);
-    if (err != cudaSuccess) {
-        if (e.state) dev_free(e.state);
-        if (e.join) cudaEventDestroy(e.join);
-        if (e.fork) cudaEventDestroy(e.fork);
-        if (e.side) cudaStreamDestroy(e.side);
-        set_cuda_error(err);
+    void* p = dev_alloc(4 * sizeof(int));
+    if (!p) return B2SR_ERR_ALLOC;
+    const cudaError_t e = cudaMemsetAsync(p, 0, 4 * sizeof(int), s);
+    if (e != cudaSuccess) {
+        set_cuda_error(e);
+        dev_free(p);
         return B2SR_ERR_CUDA;
     }
-    m->auto_side.push_back(e);
-    *out = &m->auto_side.back();
+    m->auto_state.push_back({s, p, 4 * sizeof(int)});
+    *out = static_cast<int*>(p);
     return B2SR_SUCCESS;
 }
 
@@ -540,7 +531,7 @@ static b2sr_status run_multiply(const b2sr_matrix* m, b2sr_variant v, const void
         if (dir != 0) {
             // Auto outside a capture: the device's last decision for this kind
             // is a hint.  Hinted pull: the pull alone, with the decision for the
-            // next call counted beside it on a side stream.  Otherwise classify
+            // next call counted by a few of its warps.  Otherwise classify
             // and push, and the pull is launched from the device only if the
             // push was not chosen.  Either way the result is the same bits; a
             // wrong hint costs time only.  A capture keeps the host-launched
@@ -554,27 +545,33 @@ static b2sr_status run_multiply(const b2sr_matrix* m, b2sr_variant v, const void
                 cudaGetLastError();
                 hint = nullptr;
             }
+            int* state = nullptr;
+            if (hint) {
+                st = matrix_auto_state(mm, s, &state);
+                if (st != B2SR_SUCCESS) return st;
+            }
             if (hint && reinterpret_cast<volatile int*>(hint)[kind] == 2) {
-                b2sr_matrix::AutoSide* as = nullptr;
-                st = matrix_auto_side(mm, s, &as);
-                if (st != B2SR_SUCCESS) return st;
-                B2SR_CUDA_TRY(cudaEventRecord(as->fork, s));
-                B2SR_CUDA_TRY(cudaStreamWaitEvent(as->side, as->fork, 0));
-                st = launch_direction_count(view_of(t), x, m->nt, as->state, hint_dev + kind, as->side);
-                if (st != B2SR_SUCCESS) return st;
-                B2SR_CUDA_TRY(cudaEventRecord(as->join, as->side));
-                st = rowbin_bits(*plan, view_of(m), kind, x, y, mask, accumulate, scratch, PushLink{}, true, s);
-                B2SR_CUDA_TRY(cudaStreamWaitEvent(s, as->join, 0));
-                return st;
+                DirectionCount count;
+                count.t_rowptr = t->rowptr;
+                count.state = state + 2;
+                count.hint = hint_dev + kind;
+                count.nt = m->nt;
+                count.pct = push_percent(m->T);
+                return rowbin_bits(*plan, view_of(m), kind, x, y, mask, accumulate, scratch, PushLink{}, count, true, s);
             }
             const size_t y_bytes = kind <= 1 ? (size_t)m->nb * word_bytes(m->T) : (size_t)m->nb * m->T * 4;
             st = launch_push(view_of(t), kind, dir, x, y, mask, accumulate, y_bytes, m->nt,
-                             static_cast<char*>(scratch) + pull_bytes, m->num_sms, &link,
+                             static_cast<char*>(scratch) + pull_bytes, state, m->num_sms, &link,
                              hint ? hint_dev + kind : nullptr, s);
-            if (st != B2SR_SUCCESS || dir == 2) return st;
             link.gate = hint != nullptr;
+            if (st != B2SR_SUCCESS || dir == 2) {
+                // the gate, which leaves the counters zeroed, does not follow
+                if (state) cudaMemsetAsync(state, 0, 2 * sizeof(int), s);
+                return st;
+            }
         }
-        st = rowbin_bits(*plan, view_of(m), kind, x, y, mask, accumulate, scratch, link, dir == 0, s);
+        st = rowbin_bits(*plan, view_of(m), kind, x, y, mask, accumulate, scratch, link, DirectionCount{}, dir == 0, s);
+        if (st != B2SR_SUCCESS && link.gate) cudaMemsetAsync(link.ctl, 0, 2 * sizeof(int), s);
         if (dir == 1) kernel_timer_mark(s, false);
         return st;
     }
@@ -705,14 +702,8 @@ static void free_matrix(b2sr_matrix* m) {
     m->scratch.clear();
     for (auto& e : m->spmm_state) dev_free(e.ptr);
     m->spmm_state.clear();
-    for (auto& e : m->auto_side) {
-        cudaStreamSynchronize(e.side);
-        dev_free(e.state);
-        cudaEventDestroy(e.fork);
-        cudaEventDestroy(e.join);
-        cudaStreamDestroy(e.side);
-    }
-    m->auto_side.clear();
+    for (auto& e : m->auto_state) dev_free(e.ptr);
+    m->auto_state.clear();
     if (m->auto_hint) cudaFreeHost(m->auto_hint);
     m->auto_hint = nullptr;
     for (void* p : m->retired) dev_free(p);

@@ -119,16 +119,10 @@ struct b2sr_matrix {
     std::vector<StreamScratch> spmm_state;
     // Auto direction outside stream captures: the device's last decision per
     // bit-vector kind (0 none yet, 1 push, 2 pull) in mapped host memory, read
-    // by the next call as a hint; and per stream a side stream with two events
-    // and a zeroed counter for the decision-only count beside a hinted pull.
+    // by the next call as a hint; and per stream the counters of both sides,
+    // zeroed when allocated and left zeroed by every call.
     int* auto_hint = nullptr;
-    struct AutoSide {
-        cudaStream_t stream;
-        cudaStream_t side;
-        cudaEvent_t fork, join;
-        int* state;
-    };
-    std::deque<AutoSide> auto_side;  // a deque: entries stay put while others are added
+    std::vector<StreamScratch> auto_state;
     // Buffers replaced by larger or rebuilt ones.  A CUDA graph captured
     // earlier may still hold their addresses, so they are freed only when
     // the matrix is freed.
@@ -210,11 +204,9 @@ private:
     long long max_chunks = 0, n_entries = 0;
     bool wide = false;  // 64-bit sort keys
 };
-// In-place exclusive scan of d_vals[0..n) with the total written to d_vals[n].
-// d_vals must have n + 1 entries.  d_err receives 1 if the total overflows int32.
-b2sr_status launch_exclusive_scan(int* d_vals, int n, int* d_err, cudaStream_t s);
-// The same without a wait: scratch of exclusive_scan_scratch(n) bytes, *d_err
-// left alone without an overflow.
+// In-place exclusive scan of d_vals[0..n) with the total written to d_vals[n]
+// (d_vals has n + 1 entries), asynchronous; scratch of exclusive_scan_scratch(n)
+// bytes.  *d_err is set to 1 if the total overflows int32, else left alone.
 size_t exclusive_scan_scratch(long long n);
 void exclusive_scan_async(int* d_vals, int n, int* d_err, void* scratch, cudaStream_t s);
 b2sr_status launch_pack_vec_bits(const float* x, int n, int T, void* bits, cudaStream_t s);
@@ -327,14 +319,25 @@ size_t rowbin_bits_scratch_bytes(const RowBinPlan& p, int T);
 // The push side of an auto-direction product (b2sr_push.cu) as the pull
 // kernels see it: they return at once when the push took the product.
 struct PushLink {
-    const int* ctl = nullptr;  // launch_push's counters; null: pull only
+    int* ctl = nullptr;  // launch_push's counters; null: pull only
     long long nt = 0;
     int pct = 0;  // push when the active tiles are below pct% of nt
-    bool gate = false;  // launch the pull from the device, only when chosen (not in a capture)
+    bool gate = false;  // launch the pull from the device, only when chosen, and zero ctl (not in a capture)
+};
+// Beside a pull: the tiles under x's non-zero words, counted by warps of the
+// pull kernel, and from the last of them the direction for the next call (1
+// push, 2 pull) into *hint.  state: 2 ints, zeroed, left zeroed.
+struct DirectionCount {
+    const int* t_rowptr = nullptr;  // A^T's (null: do not count)
+    int* state = nullptr;
+    int* hint = nullptr;
+    long long nt = 0;
+    int pct = 0;
 };
 // timed: kernel timer marks around the main kernel.
 b2sr_status rowbin_bits(const RowBinPlan& p, const MatView& A, int kind, const void* x, void* y, const void* mask,
-                        int accumulate, void* partials, const PushLink& link, bool timed, cudaStream_t s);
+                        int accumulate, void* partials, const PushLink& link, const DirectionCount& count, bool timed,
+                        cudaStream_t s);
 // sparse_cols: load x only for each tile's set columns (launch option gather = 3,
 // the default at T >= 16) instead of the tile-column's whole x segment.
 b2sr_status rowbin_spmv(const RowBinPlan& p, const MatView& A, const float* x, float* y, int accumulate,
@@ -355,17 +358,12 @@ __device__ __forceinline__ bool push_chosen(const int* ctl, int mode, long long 
 // Scratch bytes of launch_push: counters and the work list.
 size_t push_scratch_bytes(int nbc, long long nt);
 // mode 1 (auto) or 2 (always push); kind as rowbin_bits.  Zeroes y (y_bytes)
-// first unless accumulate.  Fills *link (counters, threshold) for the pull kernels
+// first unless accumulate.  ctl: two zeroed ints, or null for counters in the
+// scratch, zeroed first.  Fills *link (counters, threshold) for the pull kernels
 // launched after it.
 b2sr_status launch_push(const MatView& At, int kind, int mode, const void* x, void* y, const void* mask,
-                        int accumulate, size_t y_bytes, long long nt, void* scratch, int num_sms,
+                        int accumulate, size_t y_bytes, long long nt, void* scratch, int* ctl, int num_sms,
                         PushLink* link, int* hint, cudaStream_t s);
-// Auto direction: the active-tile count of x alone (no work list, y untouched)
-// into state[1] (state: 3 ints, zeroed, left zeroed), and from the last block
-// the direction (1 push, 2 pull) into *hint.
-b2sr_status launch_direction_count(const MatView& At, const void* x, long long nt, int* state, int* hint,
-                                   cudaStream_t s);
-
 // Cached texture object (uint4 texels) over [ptr, ptr + bytes), or 0 when the
 // buffer cannot back one (alignment, size).
 cudaTextureObject_t vector_texture(const void* ptr, size_t bytes);

@@ -444,8 +444,8 @@ chunk_fill_kernel(const int* __restrict__ choff, int nb, const int* __restrict__
 }
 
 // ---- exclusive scan -------------------------------------------------------------
-// Three kernels: per-block sums, a scan of the block sums in one CTA, and the
-// per-block scan with the block offset.  Sums are kept in 64 bits so an int32
+// Per-block sums, a scan of the block sums in one CTA where they are many, and
+// the per-block scan with the block offset.  Sums are kept in 64 bits so an int32
 // overflow of the total is detected instead of wrapping.
 constexpr int SCAN_THREADS = 1024;
 constexpr int SCAN_ITEMS = 4;
@@ -524,10 +524,13 @@ scan_partials_kernel(long long* __restrict__ partial, int nblocks) {
     if (threadIdx.x == 0) partial[nblocks] = carry;
 }
 
+// partial: the block sums (SUMS: every block adds up those before it), or
+// their exclusive scan.
+template <bool SUMS>
 __global__ void __launch_bounds__(SCAN_THREADS)
 scan_apply_kernel(int* __restrict__ vals, int n, const long long* __restrict__ partial,
                   int nblocks, int* __restrict__ err) {
-    __shared__ long long sh[32];
+    __shared__ long long sh[32], s_before;
     const long long base = (long long)blockIdx.x * SCAN_TILE;
     // Each thread owns SCAN_ITEMS consecutive elements.
     const long long first = base + (long long)threadIdx.x * SCAN_ITEMS;
@@ -538,8 +541,18 @@ scan_apply_kernel(int* __restrict__ vals, int n, const long long* __restrict__ p
         v[k] = (first + k < n) ? vals[first + k] : 0;
         local += v[k];
     }
+    long long before = 0;
+    if (SUMS) {
+        for (int i = threadIdx.x; i < (int)blockIdx.x; i += SCAN_THREADS) before += partial[i];
+        before = block_sum_ll(before, sh);
+        if (threadIdx.x == 0) s_before = before;
+        __syncthreads();
+        before = s_before;
+    } else {
+        before = partial[blockIdx.x];
+    }
     long long total;
-    long long ex = block_exscan_ll(local, sh, &total) + partial[blockIdx.x];
+    long long ex = block_exscan_ll(local, sh, &total) + before;
 #pragma unroll
     for (int k = 0; k < SCAN_ITEMS; ++k) {
         if (first + k < n) {
@@ -548,8 +561,8 @@ scan_apply_kernel(int* __restrict__ vals, int n, const long long* __restrict__ p
         }
         ex += v[k];
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        const long long all = partial[nblocks];
+    if ((int)blockIdx.x == nblocks - 1 && threadIdx.x == 0) {
+        const long long all = before + total;
         if (all > INT_MAX) *err = 1;
         vals[n] = (int)(all > INT_MAX ? INT_MAX : all);
     }
@@ -562,26 +575,15 @@ size_t exclusive_scan_scratch(long long n) {
 void exclusive_scan_async(int* vals, int n, int* err, void* scratch, cudaStream_t s) {
     const int nblocks = n > 0 ? (n + SCAN_TILE - 1) / SCAN_TILE : 1;
     long long* partial = static_cast<long long*>(scratch);
-    scan_reduce_kernel<<<nblocks, SCAN_THREADS, 0, s>>>(vals, n, partial);
-    scan_partials_kernel<<<1, SCAN_THREADS, 0, s>>>(partial, nblocks);
-    scan_apply_kernel<<<nblocks, SCAN_THREADS, 0, s>>>(vals, n, partial, nblocks, err);
-}
-
-b2sr_status launch_exclusive_scan(int* d_vals, int n, int* d_err, cudaStream_t s) {
-    B2SR_CUDA_TRY(cudaMemsetAsync(d_err, 0, sizeof(int), s));
-    void* partial = dev_alloc(exclusive_scan_scratch(n));
-    if (!partial) return B2SR_ERR_ALLOC;
-    exclusive_scan_async(d_vals, n, d_err, partial, s);
-    cudaError_t e = cudaGetLastError();
-    // The scratch is freed after the stream drains: the caller synchronises the
-    // stream right after the scan (it needs the total on the host).
-    cudaError_t e2 = cudaStreamSynchronize(s);
-    dev_free(partial);
-    if (e != cudaSuccess || e2 != cudaSuccess) {
-        set_cuda_error(e != cudaSuccess ? e : e2);
-        return B2SR_ERR_CUDA;
+    // one launch up to SCAN_TILE values, two while a block can add up the sums
+    // before it in a step, else three
+    if (nblocks > 1) scan_reduce_kernel<<<nblocks, SCAN_THREADS, 0, s>>>(vals, n, partial);
+    if (nblocks > SCAN_THREADS) {
+        scan_partials_kernel<<<1, SCAN_THREADS, 0, s>>>(partial, nblocks);
+        scan_apply_kernel<false><<<nblocks, SCAN_THREADS, 0, s>>>(vals, n, partial, nblocks, err);
+    } else {
+        scan_apply_kernel<true><<<nblocks, SCAN_THREADS, 0, s>>>(vals, n, partial, nblocks, err);
     }
-    return B2SR_SUCCESS;
 }
 
 // ---- host side --------------------------------------------------------------------

@@ -4,7 +4,7 @@
 // A tile-row becomes one task, or several segments when it is long; tasks are
 // listed by class (bin, or size), tile-rows ascending inside a class.  That is a
 // stable multi-way split of the tile-rows with a weight each: counts per
-// (class, block of 1024 tile-rows), one exclusive scan over all of them, and a
+// (class, block of 256 tile-rows), one exclusive scan over all of them, and a
 // second pass in which every tile-row adds its rank inside the block.  The same
 // scan places the segments' slots and the list of long rows, so a plan costs
 // one wait, for its totals.
@@ -20,7 +20,7 @@ namespace b2sr {
 
 namespace {
 
-constexpr int PLAN_ROWS = 1024;  // tile-rows per block, one per thread
+constexpr int PLAN_ROWS = 256;  // tile-rows per block, one per thread
 constexpr int PLAN_WARPS = PLAN_ROWS / 32;
 
 // What becomes of one tile-row.

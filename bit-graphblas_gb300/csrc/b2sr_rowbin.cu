@@ -647,14 +647,44 @@ struct RowBinBitsArgs {
     int warp_off[RB_BINS + 1];
     int nbc;  // x words (0: x is not read)
     int accumulate;
-    const int* push_ctl;  // auto direction: the push kernel's counters (null: always pull)
+    int* push_ctl;  // auto direction: the push kernel's counters (null: always pull)
     int push_pct;
     long long nt;
+    const int* t_rowptr;  // hinted pull: count the tiles under non-zero x words (null: do not)
+    int* count_state;     // [0] the count, [1] warps done
+    int* hint;
+    int count_warps;
 };
 
 // In auto direction the pull kernels return when the push kernel took the product.
 __device__ __forceinline__ bool pull_skipped(const RowBinBitsArgs& a) {
     return a.push_ctl != nullptr && push_chosen(a.push_ctl, 1, a.nt, a.push_pct);
+}
+
+// The first count_warps warps of a hinted pull: each adds up the tiles of A^T
+// under the non-zero words among COUNT_COLS tile-columns; the last one to finish
+// records the direction for the next call and leaves the state zeroed.  A launch
+// of its own on a second stream cost four calls for its events.
+constexpr int COUNT_COLS = 1024;
+template <int T>
+__device__ __forceinline__ void direction_count(const RowBinBitsArgs& a, int w, int lane) {
+    const auto* x = static_cast<const typename TileWord<T>::type*>(a.x);
+    int work = 0;
+#pragma unroll 4
+    for (int i = lane; i < COUNT_COLS; i += 32) {
+        const int c = w * COUNT_COLS + i;
+        if (c < a.nbc && __ldg(x + c) != 0) work += __ldg(a.t_rowptr + c + 1) - __ldg(a.t_rowptr + c);
+    }
+    work = __reduce_add_sync(FULL_MASK, work);
+    if (lane != 0) return;
+    if (work) atomicAdd(a.count_state, work);
+    __threadfence();
+    if (atomicAdd(a.count_state + 1, 1) != a.count_warps - 1) return;
+    __threadfence();
+    const long long active = atomicAdd(a.count_state, 0);
+    *reinterpret_cast<volatile int*>(a.hint) = active * 100 < a.nt * a.push_pct ? 1 : 2;
+    a.count_state[0] = 0;
+    a.count_state[1] = 0;
 }
 
 struct SemSumI32 {
@@ -749,8 +779,13 @@ __device__ __forceinline__ void wide_bits_rows(const RowBinBitsArgs& a, int task
 template <int T, int KIND>
 __global__ void __launch_bounds__(256, T <= 8 ? 8 : 1) __maxnreg__((T == 32 ? 40 : T == 16 && KIND <= 1 ? 32 : 255))
     rowbin_bits_kernel(RowBinBitsArgs a) {
-    const int warp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+    int warp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     const int lane = threadIdx.x & 31;
+    if (warp < a.count_warps) {  // 0 but in a hinted pull
+        direction_count<T>(a, warp, lane);
+        return;
+    }
+    warp -= a.count_warps;
     if (warp >= a.warp_off[RB_BINS] || pull_skipped(a)) return;
     int k = 0, woff = a.warp_off[0], toff = a.task_off[0], tend = a.task_off[1];
 #pragma unroll
@@ -869,7 +904,11 @@ __global__ void rowbin_bits_gate_kernel(RowBinBitsArgs a, unsigned blocks, unsig
     // launched behind the push kernel: wait for all of it (so the work after
     // this grid, which waits for this grid and its tail launches, follows it)
     griddep_wait();
-    if (threadIdx.x != 0 || blockIdx.x != 0 || pull_skipped(a)) return;
+    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+    const bool skipped = pull_skipped(a);
+    a.push_ctl[0] = 0;  // for the next call
+    a.push_ctl[1] = 0;
+    if (skipped) return;
     a.push_ctl = nullptr;  // the pull runs unconditionally from here
     if (blocks > 0) rowbin_bits_kernel<T, KIND><<<blocks, threads, 0, cudaStreamTailLaunch>>>(a);
     if (nlong > 0)
@@ -882,8 +921,8 @@ size_t rowbin_bits_scratch_bytes(const RowBinPlan& p, int T) {
 
 template <int T, int KIND>
 static b2sr_status run_rowbin_bits(const RowBinPlan& p, const MatView& A, const void* x, void* y, const void* mask,
-                                   int accumulate, void* partials, const PushLink& link, bool timed,
-                                   cudaStream_t s) {
+                                   int accumulate, void* partials, const PushLink& link, const DirectionCount& count,
+                                   bool timed, cudaStream_t s) {
     RowBinBitsArgs a;
     a.colind = A.colind;
     a.tiles = A.tiles;
@@ -901,7 +940,16 @@ static b2sr_status run_rowbin_bits(const RowBinPlan& p, const MatView& A, const 
     a.push_ctl = link.ctl;
     a.push_pct = link.pct;
     a.nt = link.nt;
-    const int warps = p.warp_off[RB_BINS];
+    a.t_rowptr = count.t_rowptr;
+    a.count_state = count.state;
+    a.hint = count.hint;
+    a.count_warps = 0;
+    if (count.t_rowptr) {
+        a.push_pct = count.pct;
+        a.nt = count.nt;
+        a.count_warps = (a.nbc + COUNT_COLS - 1) / COUNT_COLS;
+    }
+    const int warps = p.warp_off[RB_BINS] + a.count_warps;
     int launches = 0;
     const unsigned fix_blocks = (unsigned)((fixup_warps(p.nlong, p.nlong_short) + 7) / 8);
     if (link.ctl && link.gate) {
@@ -935,24 +983,25 @@ static b2sr_status run_rowbin_bits(const RowBinPlan& p, const MatView& A, const 
 
 template <int T>
 static b2sr_status bits_kind(int kind, const RowBinPlan& p, const MatView& A, const void* x, void* y,
-                             const void* mask, int accumulate, void* partials, const PushLink& link, bool timed,
-                             cudaStream_t s) {
+                             const void* mask, int accumulate, void* partials, const PushLink& link, const DirectionCount& count,
+                             bool timed, cudaStream_t s) {
     switch (kind) {
-        case 0: return run_rowbin_bits<T, 0>(p, A, x, y, mask, accumulate, partials, link, timed, s);
-        case 1: return run_rowbin_bits<T, 1>(p, A, x, y, mask, accumulate, partials, link, timed, s);
-        case 2: return run_rowbin_bits<T, 2>(p, A, x, y, mask, accumulate, partials, link, timed, s);
-        case 3: return run_rowbin_bits<T, 3>(p, A, x, y, mask, accumulate, partials, link, timed, s);
+        case 0: return run_rowbin_bits<T, 0>(p, A, x, y, mask, accumulate, partials, link, count, timed, s);
+        case 1: return run_rowbin_bits<T, 1>(p, A, x, y, mask, accumulate, partials, link, count, timed, s);
+        case 2: return run_rowbin_bits<T, 2>(p, A, x, y, mask, accumulate, partials, link, count, timed, s);
+        case 3: return run_rowbin_bits<T, 3>(p, A, x, y, mask, accumulate, partials, link, count, timed, s);
     }
     return B2SR_ERR_INVALID_VALUE;
 }
 
 b2sr_status rowbin_bits(const RowBinPlan& p, const MatView& A, int kind, const void* x, void* y, const void* mask,
-                        int accumulate, void* partials, const PushLink& link, bool timed, cudaStream_t s) {
+                        int accumulate, void* partials, const PushLink& link, const DirectionCount& count, bool timed,
+                        cudaStream_t s) {
     switch (A.T) {
-        case 4: return bits_kind<4>(kind, p, A, x, y, mask, accumulate, partials, link, timed, s);
-        case 8: return bits_kind<8>(kind, p, A, x, y, mask, accumulate, partials, link, timed, s);
-        case 16: return bits_kind<16>(kind, p, A, x, y, mask, accumulate, partials, link, timed, s);
-        case 32: return bits_kind<32>(kind, p, A, x, y, mask, accumulate, partials, link, timed, s);
+        case 4: return bits_kind<4>(kind, p, A, x, y, mask, accumulate, partials, link, count, timed, s);
+        case 8: return bits_kind<8>(kind, p, A, x, y, mask, accumulate, partials, link, count, timed, s);
+        case 16: return bits_kind<16>(kind, p, A, x, y, mask, accumulate, partials, link, count, timed, s);
+        case 32: return bits_kind<32>(kind, p, A, x, y, mask, accumulate, partials, link, count, timed, s);
     }
     return B2SR_ERR_INVALID_VALUE;
 }

@@ -508,20 +508,64 @@ int spmm_rows_seg(int T, long long nt, int num_sms) {
     return (int)std::min(8192LL, std::max(128LL, visits * 30 / (100 * warps)));
 }
 
-// Set bits of every tile-row: one warp per tile-row (grid-stride), popc of
-// its tiles' 32-bit words (the unused bits of a tile are zero).
-__global__ void tile_row_bits_kernel(const int* __restrict__ rowptr, const uint32_t* __restrict__ words, int nb,
-                                     int wpt, long long* __restrict__ bits) {
+// Set bits of every tile-row, into zeroed bits[nb].  A warp takes 512 tiles in
+// a row, 32 at a time (one per lane, its words with the widest loads), finds the
+// tile-row of each once and adds up the lanes of one tile-row before it adds to
+// bits[]: balanced whatever the row lengths (a warp per tile-row waited 38 us
+// for the hubs of R-MAT scale 16; 4 us this way).  rowptr may be anything: a
+// tile's row is searched in [0, nb).
+constexpr int BITS_TILES = 512;
+template <int T>
+__global__ void __launch_bounds__(256)
+tile_row_bits_kernel(const int* __restrict__ rowptr, const void* __restrict__ tiles, int nb, int nt,
+                     unsigned long long* __restrict__ bits) {
     const int lane = threadIdx.x & 31;
-    const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
-    for (long long r = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < nb; r += nwarps) {
-        const long long b = (long long)rowptr[r] * wpt, e = (long long)rowptr[r + 1] * wpt;
-        long long c = 0;
-        for (long long k = b + lane; k < e; k += 32) c += __popc(__ldg(words + k));
+    const long long first = (((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * BITS_TILES;
+    if (first >= nt) return;  // warp-uniform
+    const int end = (int)min(first + BITS_TILES, (long long)nt);
+    auto row_of = [&](int j) {  // the last tile-row that starts at or before tile j
+        int lo = 0, hi = nb;
+        while (hi - lo > 1) {
+            const int mid = lo + ((hi - lo) >> 1);
+            if (rowptr[mid] <= j) lo = mid;
+            else hi = mid;
+        }
+        return lo;
+    };
+    int row = row_of((int)first), next = rowptr[row + 1];  // warp-uniform, and where it ends
+    unsigned sum = 0;                                         // this lane's bits of `row`
+    for (int j0 = (int)first; j0 < end; j0 += 32) {
+        const int j = j0 + lane;
+        unsigned c = 0;
+        if (j < end) {
+            if constexpr (T == 8) {
+                const uint2 v = __ldg(static_cast<const uint2*>(tiles) + j);
+                c = __popc(v.x) + __popc(v.y);
+            } else {
+                const uint4* p = static_cast<const uint4*>(tiles) + (size_t)j * (T * T / 128);
 #pragma unroll
-        for (int o = 16; o; o >>= 1) c += __shfl_xor_sync(FULL_MASK, c, o);
-        if (lane == 0) bits[r] = c;
+                for (int q = 0; q < T * T / 128; ++q) {
+                    const uint4 v = __ldg(p + q);
+                    c += __popc(v.x) + __popc(v.y) + __popc(v.z) + __popc(v.w);
+                }
+            }
+        }
+        if (min(j0 + 32, end) <= next) {  // all of one tile-row
+            sum += c;
+            continue;
+        }
+        // the step crosses tile-rows: the open one, then a tile-row per lane
+        sum += j < next ? c : 0u;
+        sum = __reduce_add_sync(FULL_MASK, sum);
+        if (lane == 0 && sum) atomicAdd(bits + row, (unsigned long long)sum);
+        const int mine = j >= next && j < end ? row_of(j) : -1;
+        row = row_of(min(j0 + 31, end - 1));
+        next = rowptr[row + 1];
+        if (mine >= 0 && mine != row && c) atomicAdd(bits + mine, (unsigned long long)c);
+        sum = mine == row ? c : 0u;
     }
+    sum = __reduce_add_sync(FULL_MASK, sum);
+    if (lane == 0 && sum) atomicAdd(bits + row, (unsigned long long)sum);
 }
 
 b2sr_status spmm_rows_plan_create(const int* d_rowptr, const void* d_tiles, int nb, int nt, long long nnz, int T,
@@ -545,9 +589,17 @@ b2sr_status spmm_rows_plan_create(const int* d_rowptr, const void* d_tiles, int 
     if (T >= 8 && nb > 0) {
         d_bits = static_cast<long long*>(dev_alloc(sizeof(long long) * (size_t)nb));
         if (!d_bits) return B2SR_ERR_ALLOC;
-        const long long blocks = std::min<long long>(((long long)nb * 32 + 255) / 256, 65535LL * 8);
-        tile_row_bits_kernel<<<(unsigned)blocks, 256, 0, s>>>(d_rowptr, static_cast<const uint32_t*>(d_tiles), nb,
-                                                                T * T / 32, d_bits);
+        const cudaError_t e = cudaMemsetAsync(d_bits, 0, sizeof(long long) * (size_t)nb, s);
+        if (e != cudaSuccess) {
+            set_cuda_error(e);
+            dev_free(d_bits);
+            return B2SR_ERR_CUDA;
+        }
+        const unsigned blocks = (unsigned)(((long long)nt + BITS_TILES * 8 - 1) / (BITS_TILES * 8));
+        auto* bits = reinterpret_cast<unsigned long long*>(d_bits);
+        if (nt > 0 && T == 8) tile_row_bits_kernel<8><<<blocks, 256, 0, s>>>(d_rowptr, d_tiles, nb, nt, bits);
+        if (nt > 0 && T == 16) tile_row_bits_kernel<16><<<blocks, 256, 0, s>>>(d_rowptr, d_tiles, nb, nt, bits);
+        if (nt > 0 && T == 32) tile_row_bits_kernel<32><<<blocks, 256, 0, s>>>(d_rowptr, d_tiles, nb, nt, bits);
         rule.row_bits = d_bits;
         const long long warps = (long long)std::max(num_sms, 1) * ROWS_BLOCKS * ROWS_WARPS;
         rule.seg_bits = std::max(1024LL, nnz * 7 / (10 * warps));
