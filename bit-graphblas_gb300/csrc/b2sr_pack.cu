@@ -8,7 +8,7 @@
 //
 //   1. validate the CSR, an entry per thread (which also counts duplicates, so
 //      the number of set bits is known without reading the tiles);
-//   2. cut every tile-row into chunks of about CHUNK_ENTRIES entries;
+//   2. cut every tile-row into chunks of about 400 (T = 4) or 320 entries;
 //   3. a warp per chunk sorts the chunk's entries by (tile-column, row, column)
 //      in registers, writes the sorted keys and counts the tiles;
 //   4. scans give the tile-row pointer and the tile count (the one value the
@@ -101,17 +101,20 @@ validate_entries_kernel(const int* __restrict__ colind, int ncols, int nnz, cons
 }
 
 // ---- chunks ---------------------------------------------------------------------
-// A tile-row of L entries has ceil(L / CHUNK_ENTRIES) chunks (none when empty),
+// A tile-row of L entries has ceil(L / chunk_entries) chunks (none when empty),
 // cut at the tile-columns of every q-th entry of its longest row, so a chunk
-// covers a range of tile-columns and holds about CHUNK_ENTRIES entries.  A
+// covers a range of tile-columns and holds about chunk_entries entries.  A
 // warp sorts up to CHUNK_CAP of them; rows that fill the range unevenly can
-// exceed that (R-MAT scale 18: 0 - 0.5% of the chunks, at 440 entries up to
-// 1.7%), and dense tiles or duplicates do: such a chunk is merged by T lanes
-// instead.  A tile-row of at most CHUNK_CAP entries is one chunk.
+// exceed that, and dense tiles or duplicates do: such a chunk is merged by T
+// lanes instead, one tile-column at a time, so a few of them set the time.
+// 400 at T = 4 and 320 above: packing R-MAT scale 16 at T = 8 takes 213 us with
+// 320, 247 with 400 and 286 with 450 (scale 18: 328, 342, 437), scale 20 at
+// T = 4 827, 798 and 900.  A tile-row of at most CHUNK_CAP entries is one chunk.
 constexpr int CHUNK_CAP = 512;
-constexpr int CHUNK_ENTRIES = 400;
-__host__ __device__ __forceinline__ int chunks_of(int entries) {
-    return entries == 0 ? 0 : entries <= CHUNK_CAP ? 1 : (entries + CHUNK_ENTRIES - 1) / CHUNK_ENTRIES;
+__host__ __device__ constexpr int chunk_entries(int T) { return T == 4 ? 400 : 320; }
+__host__ __device__ __forceinline__ int chunks_of(int entries, int T) {
+    const int per = chunk_entries(T);
+    return entries == 0 ? 0 : entries <= CHUNK_CAP ? 1 : (entries + per - 1) / per;
 }
 
 // Chunks of every tile-row, and their sums per SCAN_TILE tile-rows.
@@ -122,7 +125,7 @@ __global__ void chunk_plan_kernel(const int* __restrict__ rowptr, int nrows, int
     int n = 0;
     if (info->flag == 0) {
         const long long r0 = tr * T, r1 = r0 + T < nrows ? r0 + T : nrows;
-        n = chunks_of(rowptr[r1] - rowptr[r0]);
+        n = chunks_of(rowptr[r1] - rowptr[r0], T);
     }
     nch[tr] = n;
 }
@@ -661,7 +664,7 @@ b2sr_status PackJob::count(const int* rowptr, const int* colind, int nrows, int 
     }
     wide = !(T == 4 ? key_fits_32<4>(ncols) : T == 8 ? key_fits_32<8>(ncols) : T == 16 ? key_fits_32<16>(ncols)
                                                                                    : key_fits_32<32>(ncols));
-    max_chunks = nb + nnz / CHUNK_ENTRIES + 1;  // sum over tile-rows of ceil(entries / CHUNK_ENTRIES)
+    max_chunks = nb + nnz / chunk_entries(T) + 1;  // sum over tile-rows of ceil(entries / chunk_entries)
     n_entries = nnz;
     const size_t key = wide ? 8 : 4;
     scratch = dev_alloc(Layout(nullptr, nb, max_chunks, nnz, key).bytes);
