@@ -661,7 +661,7 @@ __device__ __forceinline__ bool pull_skipped(const RowBinBitsArgs& a) {
     return a.push_ctl != nullptr && push_chosen(a.push_ctl, 1, a.nt, a.push_pct);
 }
 
-// The first count_warps warps of a hinted pull: each adds up the tiles of A^T
+// The last count_warps warps of a hinted pull: each adds up the tiles of A^T
 // under the non-zero words among COUNT_COLS tile-columns; the last one to finish
 // records the direction for the next call and leaves the state zeroed.  A launch
 // of its own on a second stream cost four calls for its events.
@@ -779,14 +779,14 @@ __device__ __forceinline__ void wide_bits_rows(const RowBinBitsArgs& a, int task
 template <int T, int KIND>
 __global__ void __launch_bounds__(256, T <= 8 ? 8 : 1) __maxnreg__((T == 32 ? 40 : T == 16 && KIND <= 1 ? 32 : 255))
     rowbin_bits_kernel(RowBinBitsArgs a) {
-    int warp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+    const int warp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     const int lane = threadIdx.x & 31;
-    if (warp < a.count_warps) {  // 0 but in a hinted pull
-        direction_count<T>(a, warp, lane);
+    if (warp >= a.warp_off[RB_BINS]) {
+        const int w = warp - a.warp_off[RB_BINS];
+        if (w < a.count_warps) direction_count<T>(a, w, lane);  // none but in a hinted pull
         return;
     }
-    warp -= a.count_warps;
-    if (warp >= a.warp_off[RB_BINS] || pull_skipped(a)) return;
+    if (pull_skipped(a)) return;
     int k = 0, woff = a.warp_off[0], toff = a.task_off[0], tend = a.task_off[1];
 #pragma unroll
     for (int kk = 1; kk < RB_BINS; ++kk) {
