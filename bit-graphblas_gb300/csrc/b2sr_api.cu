@@ -669,7 +669,7 @@ static b2sr_status run_spmm_api(const b2sr_matrix* m, const V* X, int k, long lo
         if (st != B2SR_SUCCESS) return st;
         void* state = nullptr;
         Scratch state_fallback;
-        st = matrix_spmm_state(m, s, spmm_rows_state_bytes(m->spmm_rows), &state, state_fallback);
+        st = matrix_spmm_state(m, s, spmm_rows_state_bytes(), &state, state_fallback);
         if (st != B2SR_SUCCESS) return st;
         return spmm_rows_launch<V>(view_of(m), m->spmm_rows, X, ldx, Y, ldy, k,
                                    m->shapes[B2SR_BIN_FULL_FULL].rhs_block, accumulate, scratch,

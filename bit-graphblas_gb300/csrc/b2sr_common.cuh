@@ -69,9 +69,8 @@ struct RowBinPlan {
 struct SpmmRowsPlan {
     int4* d_tasks = nullptr;
     int4* d_long = nullptr;      // (tile-row, first slot, slots, 0)
-    int* d_slot_long = nullptr;  // long row of every slot
     int ntasks = 0, nlong = 0, nslots = 0;
-    int groups = 1;              // row groups per tile-row (T / rows per task)
+    int nnarrow = 0;  // long rows of few slots, listed first in d_long
 };
 
 // Per-variant cached launch data of a matrix: the grid and the merge-path
@@ -113,9 +112,8 @@ struct b2sr_matrix {
     };
     std::mutex scratch_mu;
     std::vector<StreamScratch> scratch;
-    // Per-stream counters of the row-task SpMM kernel (work queue, long-row
-    // arrivals): zeroed when allocated, left zeroed by every launch, and
-    // used by nothing else.
+    // Per-stream counters of the row-task SpMM kernel's work queue: zeroed when
+    // allocated, left zeroed by every launch, and used by nothing else.
     std::vector<StreamScratch> spmm_state;
     // Auto direction outside stream captures: the device's last decision per
     // bit-vector kind (0 none yet, 1 push, 2 pull) in mapped host memory, read
@@ -230,15 +228,17 @@ constexpr int PLAN_CLASSES = 64;
 // row_bits also hold at most about seg_bits set bits each.  Tasks are listed by
 // class, tile-rows ascending inside a class:
 //   BINS    nbins bins by tile count (bin b: up to unit << b tiles), the last
-//           bin first; long rows of at most narrow_slots slots listed first
+//           bin first
 //   TWO     tasks of at least a quarter of seg, then the rest
 //   LENGTH  longest first, in four classes per octave
 //   BITS    most set bits first, in two classes per octave
+// Long rows of at most narrow_slots slots are listed before the others.
 struct PlanRule {
     enum Kind { BINS, TWO, LENGTH, BITS } kind;
     int seg;
     int classes;
     int unit = 0, nbins = 0, narrow_slots = 0;
+    int whole = 0, whole_bits = 0;  // tile-rows with no more tiles / set bits than this are not cut
     const long long* row_bits = nullptr;
     long long seg_bits = 0;
 };
@@ -248,9 +248,8 @@ struct PlanBounds {
 struct PlanOut {
     int4* tasks;     // (tile-row, first tile, end tile, slot or -1)
     int4* longs;     // (tile-row, first slot, slots, 0)
-    int* slot_long;  // long row of every slot (null: not wanted)
     int* info;
-    int cap_tasks, cap_long, cap_slots;
+    int cap_tasks, cap_long;
 };
 struct PlanTotals {
     int tasks = 0, longs = 0, narrow = 0, slots = 0;
@@ -260,7 +259,7 @@ struct PlanTotals {
 PlanBounds plan_bounds(const PlanRule& r, int nb, long long nt, long long bits);
 // Fills the arrays (of those sizes).  Synchronizes `s`.
 b2sr_status build_plan(const PlanRule& rule, const int* rowptr, int nb, const PlanBounds& cap, int4* tasks, int4* longs,
-                       int* slot_long, PlanTotals* totals, cudaStream_t s);
+                       PlanTotals* totals, cudaStream_t s);
 
 // ---- multiply (b2sr_spmv.cu) --------------------------------------------------
 struct MatView {
@@ -302,7 +301,7 @@ b2sr_status spmm_rows_plan_create(const int* d_rowptr, const void* d_tiles, int 
                                   int num_sms, SpmmRowsPlan* out, cudaStream_t s);
 void spmm_rows_plan_free(SpmmRowsPlan* p);
 size_t spmm_rows_scratch_bytes(const SpmmRowsPlan& p, int T, int elem_bytes, int k);
-size_t spmm_rows_state_bytes(const SpmmRowsPlan& p);
+size_t spmm_rows_state_bytes();
 template <typename V>
 b2sr_status spmm_rows_launch(const MatView& A, const SpmmRowsPlan& p, const V* X, long long ldx, V* Y,
                              long long ldy, int k, int rhs_block, int accumulate, void* scratch, int* state,

@@ -45,7 +45,7 @@ __device__ __forceinline__ RowTasks row_tasks(const PlanRule& r, const int* __re
     if (i >= nb) return t;
     t.b0 = rowptr[i];
     t.m = rowptr[i + 1] - t.b0;
-    t.nseg = t.m > r.seg ? (t.m - 1) / r.seg + 1 : 1;
+    t.nseg = t.m > max(r.seg, r.whole) ? (t.m - 1) / r.seg + 1 : 1;
     if (r.kind == PlanRule::BINS) {
         int b = 0;
         while (b < r.nbins - 1 && t.m > (r.unit << b)) ++b;
@@ -56,9 +56,10 @@ __device__ __forceinline__ RowTasks row_tasks(const PlanRule& r, const int* __re
     long long bits = 0;
     if (r.row_bits) {
         bits = r.row_bits[i];
-        const long long by_bits = (bits + r.seg_bits - 1) / r.seg_bits;
+        const long long by_bits = bits > r.whole_bits ? (bits + r.seg_bits - 1) / r.seg_bits : 1;
         t.nseg = (int)min((long long)max(t.m, 1), max((long long)t.nseg, by_bits));
     }
+    t.narrow = t.nseg <= r.narrow_slots;
     const int len = (t.m + t.nseg - 1) / t.nseg;  // of a segment
     if (r.kind == PlanRule::TWO) t.cls = 4LL * len >= r.seg ? 0 : 1;
     else if (r.kind == PlanRule::LENGTH) t.cls = size_class<4>(len);
@@ -142,15 +143,15 @@ plan_emit_kernel(PlanRule rule, const int* __restrict__ rowptr, int nb, int nblo
     auto at = [&](int k) { return offs[(long long)k * nblocks + blockIdx.x]; };
     const int first_slot = offs[(long long)(rule.classes + C_SLOTS) * nblocks];
     const int first_long = offs[(long long)(rule.classes + C_NARROW) * nblocks];
-    int task = 0, slot = -1, lr = 0;
+    int task = 0, slot = -1;
     if (on) task = at(t.cls) + wcnt[warp][t.cls] + rank;
     if (cut) {
         slot = at(rule.classes + C_SLOTS) - first_slot + wextra[warp][C_SLOTS] + pre[C_SLOTS];
         const int x = t.narrow ? C_NARROW : C_LONG;
-        lr = at(rule.classes + x) - first_long + wextra[warp][x] + pre[x];
+        const int lr = at(rule.classes + x) - first_long + wextra[warp][x] + pre[x];
         if (lr < out.cap_long) out.longs[lr] = make_int4(i, slot, t.nseg, 0);
     }
-    auto emit = [&](int row, int b0, int m, int nseg, int task, int slot, int lr, int q) {
+    auto emit = [&](int row, int b0, int m, int nseg, int task, int slot, int q) {
         int t0, t1;
         if (rule.kind == PlanRule::BINS) {  // whole segments, the last one shorter
             t0 = b0 + q * rule.seg;
@@ -160,18 +161,16 @@ plan_emit_kernel(PlanRule rule, const int* __restrict__ rowptr, int nb, int nblo
             t1 = b0 + (int)((long long)m * (q + 1) / nseg);
         }
         if (task + q < out.cap_tasks) out.tasks[task + q] = make_int4(row, t0, t1, slot < 0 ? -1 : slot + q);
-        if (slot >= 0 && out.slot_long && slot + q < out.cap_slots) out.slot_long[slot + q] = lr;
     };
     if (on && t.nseg <= 4)
-        for (int q = 0; q < t.nseg; ++q) emit(i, t.b0, t.m, t.nseg, task, slot, lr, q);
+        for (int q = 0; q < t.nseg; ++q) emit(i, t.b0, t.m, t.nseg, task, slot, q);
     // long rows by the whole warp
     for (unsigned c = __ballot_sync(FULL_MASK, on && t.nseg > 4); c; c &= c - 1) {
         const int l = __ffs(c) - 1;
         const int row = __shfl_sync(FULL_MASK, i, l), b0 = __shfl_sync(FULL_MASK, t.b0, l),
                   m = __shfl_sync(FULL_MASK, t.m, l), nseg = __shfl_sync(FULL_MASK, t.nseg, l),
-                  tk = __shfl_sync(FULL_MASK, task, l), sl = __shfl_sync(FULL_MASK, slot, l),
-                  ll = __shfl_sync(FULL_MASK, lr, l);
-        for (int q = lane; q < nseg; q += 32) emit(row, b0, m, nseg, tk, sl, ll, q);
+                  tk = __shfl_sync(FULL_MASK, task, l), sl = __shfl_sync(FULL_MASK, slot, l);
+        for (int q = lane; q < nseg; q += 32) emit(row, b0, m, nseg, tk, sl, q);
     }
 }
 
@@ -186,7 +185,7 @@ PlanBounds plan_bounds(const PlanRule& r, int nb, long long nt, long long bits) 
 }
 
 b2sr_status build_plan(const PlanRule& rule, const int* rowptr, int nb, const PlanBounds& cap, int4* tasks, int4* longs,
-                       int* slot_long, PlanTotals* totals, cudaStream_t s) {
+                       PlanTotals* totals, cudaStream_t s) {
     const int nblocks = (nb + PLAN_ROWS - 1) / PLAN_ROWS;
     const long long n = (long long)(rule.classes + C_EXTRA) * nblocks;
     if (n > INT_MAX || cap.tasks > INT_MAX || cap.slots > INT_MAX) return B2SR_ERR_OVERFLOW;
@@ -204,7 +203,7 @@ b2sr_status build_plan(const PlanRule& rule, const int* rowptr, int nb, const Pl
     if (e == cudaSuccess && nb > 0) {
         plan_count_kernel<<<nblocks, PLAN_ROWS, 0, s>>>(rule, rowptr, nb, nblocks, hist);
         exclusive_scan_async(hist, (int)n, err, scratch + sizeof(int) * info_ints + hist_bytes, s);
-        const PlanOut out{tasks, longs, slot_long, info, (int)cap.tasks, (int)cap.longs, (int)cap.slots};
+        const PlanOut out{tasks, longs, info, (int)cap.tasks, (int)cap.longs};
         plan_emit_kernel<<<nblocks, PLAN_ROWS, 0, s>>>(rule, rowptr, nb, nblocks, hist, out);
         e = cudaGetLastError();
     }

@@ -525,7 +525,7 @@ b2sr_status rowbin_plan_create(const int* d_rowptr, int nb, int nt, int T, bool 
     if (!p.d_tasks) return B2SR_ERR_ALLOC;
     p.d_long = p.d_tasks + cap.tasks;
     PlanTotals t;
-    const b2sr_status st = build_plan(rule, d_rowptr, nb, cap, p.d_tasks, p.d_long, nullptr, &t, s);
+    const b2sr_status st = build_plan(rule, d_rowptr, nb, cap, p.d_tasks, p.d_long, &t, s);
     if (st != B2SR_SUCCESS) {
         dev_free(p.d_tasks);
         return st;

@@ -6,13 +6,12 @@
 // Plan (once per matrix, b2sr_plan.cu): one task per tile-row; a tile-row
 // longer than spmm_rows_seg() tiles (a share of one resident warp's part of all
 // the tiles), or at T >= 8 with more than such a share of the set bits, is cut
-// into near-equal segments whose partial rows go to slots.  The warp that
-// finishes a row's last segment (a per-row arrival counter) adds the row's
-// slots in segment order and writes Y, so a multiply is one launch.  Warps take
+// into near-equal segments whose partial rows go to slots, which a second
+// kernel adds in segment order.  Warps take
 // (column block, task, row group) work items from a device queue (an atomic
 // counter); long tasks are handed out first, so the queue ends on short ones
 // (R-MAT hubs sit all over the vertex range, and in row order the last items
-// could be the longest).  The queue and arrival counters live in a zeroed
+// could be the longest).  The queue's counters live in a zeroed
 // per-(matrix, stream) state buffer that the kernel's last warp leaves zeroed
 // again, so no launch needs a memset.
 //
@@ -100,22 +99,8 @@ __device__ __forceinline__ void rows_add_all(V (&acc)[VEC], V (&v)[N][VEC]) {
     }
 }
 
-// rows_load through L2 only (data written by other SMs in this launch)
-template <typename V, int VEC, bool FULL, int STR>
-__device__ __forceinline__ void rows_load_l2(V (&out)[VEC], const V* p, int nvalid) {
-    if constexpr (FULL) {
-        using VT = typename RowsVec<V, VEC>::type;
-        const VT v = __ldcg(reinterpret_cast<const VT*>(p));
-        const V* e = reinterpret_cast<const V*>(&v);
-#pragma unroll
-        for (int i = 0; i < VEC; ++i) out[i] = e[i];
-    } else {
-#pragma unroll
-        for (int i = 0; i < VEC; ++i) out[i] = i < nvalid ? __ldcg(p + i * STR) : V(0);
-    }
-}
-
-template <typename V, int VEC, bool FULL, int STR>
+// STREAM: evict-first, for rows that nothing reads soon.
+template <typename V, int VEC, bool FULL, int STR, bool STREAM = false>
 __device__ __forceinline__ void rows_store(V* p, const V (&v)[VEC], int nvalid, bool accumulate) {
     if constexpr (FULL) {
         using VT = typename RowsVec<V, VEC>::type;
@@ -131,7 +116,8 @@ __device__ __forceinline__ void rows_store(V* p, const V (&v)[VEC], int nvalid, 
 #pragma unroll
             for (int i = 0; i < VEC; ++i) e[i] = v[i];
         }
-        *q = o;
+        if (STREAM) __stcs(q, o);
+        else *q = o;
     } else {
 #pragma unroll
         for (int i = 0; i < VEC; ++i)
@@ -205,19 +191,12 @@ struct SpmmRowsArgs {
     int ncb;  // column blocks of (32 / IPW) * VEC columns
     const int4* tasks;  // (tile-row, first tile, end tile, slot or -1)
     int ntasks;
-    int* state;   // [0] queue counter, [1] warps done, [2 + i*G + g] segments done of long row i, row group g
+    int* state;   // [0] queue counter, [1] warps done
     const int4* long_rows;  // (tile-row, first slot, slots, 0)
-    const int* slot_long;   // long row of every slot
     V* partials;  // slot x T x k
     int accumulate;
 };
 
-// The warp that finished the last segment of long row lr's row group (rows
-// r0 .. r0+R-1 of its tile-row): those Y rows (+)= the row's slots added in
-// segment order, over all k columns (every column block of the group has
-// arrived); sub-group `sub` takes rows r0+sub, r0+sub+IPW, ...  SL slots in
-// flight (the main loop needs the registers), added in slot order; no unrolling of the outer loops (an out-of-line call
-// measured slower).
 // First column of a lane in column block cb, and how many columns it has there.
 template <int VEC, int LPI, bool FULL>
 __device__ __forceinline__ int rows_col(int cb, int lane, int k, int& nvalid) {
@@ -226,47 +205,66 @@ __device__ __forceinline__ int rows_col(int cb, int lane, int k, int& nvalid) {
     return col;
 }
 
-template <int T, int IPW, int VEC, bool FULL, typename V>
-__device__ __forceinline__ void rows_long_reduce(const SpmmRowsArgs<V>& a, int lr, int lane, int r0) {
-    constexpr int LPI = 32 / IPW;
-    constexpr int R = ROWS_R;
-    constexpr int SL = 2;
-    const int sub = lane / LPI;
+// Long rows: Y row (+)= the row's slots.  A unit is one of a long row's T rows
+// and 32 lanes of columns.  Rows of at most NARROW_SLOTS slots (listed first)
+// take a warp per unit, slots in segment order; the others a block per unit,
+// whose warps add a share of the slots each, in order, and then the shares in
+// order.  Launched behind the main kernel.  (The warp that finished a row's last
+// segment used to add its slots there, one tile-row at a time and two slots in
+// flight beside the main loop's registers: with as many segments as small
+// graphs need, hubs waited for it.)
+constexpr int NARROW_SLOTS = 32;
+template <int T, bool FULL, typename V>
+__global__ void __launch_bounds__(ROWS_WARPS * 32, 4)
+rows_fixup_kernel(SpmmRowsArgs<V> a, int nnarrow, int narrow_blocks, int ncb) {
+    constexpr int VEC = FULL ? 16 / (int)sizeof(V) : 1, SL = 8;
+    __shared__ V s_part[ROWS_WARPS][32 * VEC];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const bool alone = (int)blockIdx.x < narrow_blocks;  // block-uniform
+    long long unit = alone ? (long long)blockIdx.x * ROWS_WARPS + warp : (long long)blockIdx.x - narrow_blocks;
+    const int cb = (int)(unit % ncb), r = (int)(unit / ncb % T);
+    long long lr = unit / ncb / T;
+    if (alone && lr >= nnarrow) return;  // a block's last warps: nothing of theirs to wait for
+    if (!alone) lr += nnarrow;
     const int4 L = __ldg(a.long_rows + lr);
+    int nvalid;
+    const int col = rows_col<VEC, 32, FULL>(cb, lane, a.k, nvalid);
+    griddep_wait();  // the main kernel's slots
+    const V* src = a.partials + ((long long)L.y * T + r) * a.k + col;
     const long long stride = (long long)T * a.k;
-#pragma unroll 1
-    for (int cb = 0; cb < a.ncb; ++cb) {
-        int nvalid;
-        const int col = rows_col<VEC, LPI, FULL>(cb, lane, a.k, nvalid);
-        if (nvalid == 0) continue;
-#pragma unroll 1
-        for (int r = r0 + sub; r < r0 + R; r += IPW) {
-            const V* src = a.partials + ((long long)L.y * T + r) * a.k + col;
-            V tot[VEC];
+    const int end = alone ? L.z : (int)((long long)L.z * (warp + 1) / ROWS_WARPS);
+    V tot[VEC];
 #pragma unroll
-            for (int e = 0; e < VEC; ++e) tot[e] = V(0);
-            int q = 0;
-#pragma unroll 1
-            for (; q + SL - 1 < L.z; q += SL) {
-                V v[SL][VEC];
+    for (int e = 0; e < VEC; ++e) tot[e] = V(0);
+    if (nvalid > 0) {
+        int q = alone ? 0 : (int)((long long)L.z * warp / ROWS_WARPS);
+        for (; q + SL <= end; q += SL) {
+            V v[SL][VEC];
 #pragma unroll
-                for (int u = 0; u < SL; ++u) rows_load_l2<V, VEC, FULL, LPI>(v[u], src + (q + u) * stride, nvalid);
+            for (int u = 0; u < SL; ++u) rows_load<V, VEC, FULL, 32>(v[u], src + (q + u) * stride, nvalid);
 #pragma unroll
-                for (int u = 0; u < SL; ++u)
+            for (int u = 0; u < SL; ++u) rows_add<V, VEC>(tot, v[u]);
+        }
+        if (q < end) {  // the rest, also in flight together
+            V v[SL][VEC];
 #pragma unroll
-                    for (int e = 0; e < VEC; ++e) tot[e] += v[u][e];
-            }
-#pragma unroll 1
-            for (; q < L.z; ++q) {
-                V v0[VEC];
-                rows_load_l2<V, VEC, FULL, LPI>(v0, src + q * stride, nvalid);
+            for (int u = 0; u < SL; ++u) rows_load<V, VEC, FULL, 32>(v[u], src + (min(q + u, end - 1)) * stride, nvalid);
 #pragma unroll
-                for (int e = 0; e < VEC; ++e) tot[e] += v0[e];
-            }
-            rows_store<V, VEC, FULL, LPI>(a.Y + ((long long)L.x * T + r) * a.ldy + col, tot, nvalid,
-                                          a.accumulate != 0);
+            for (int u = 0; u < SL; ++u)
+                if (q + u < end) rows_add<V, VEC>(tot, v[u]);
         }
     }
+    if (!alone) {
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) s_part[warp][e * 32 + lane] = tot[e];
+        __syncthreads();
+        if (warp != 0) return;
+        for (int w = 1; w < ROWS_WARPS; ++w)
+#pragma unroll
+            for (int e = 0; e < VEC; ++e) tot[e] += s_part[w][e * 32 + lane];
+    }
+    if (nvalid > 0)
+        rows_store<V, VEC, FULL, 32>(a.Y + ((long long)L.x * T + r) * a.ldy + col, tot, nvalid, a.accumulate != 0);
 }
 
 // A lane holds VEC columns, LPI = 32/IPW lanes a column block of LPI*VEC
@@ -274,9 +272,14 @@ __device__ __forceinline__ void rows_long_reduce(const SpmmRowsArgs<V>& a, int l
 // two X rows of 16 lanes x 16 bytes).  FULL: 16 bytes of neighbouring columns
 // per lane, every vector whole and aligned.  Otherwise rows_width() picks as
 // few scalar columns per lane as cover k.
+// STREAM (whole-warp vector rows, k > 64 FP32, of a matrix with long rows):
+// colind and Y pass through L2 evict-first, which leaves it to the X rows that
+// the hubs reuse: R-MAT scale 20, k = 128 2040 -> 2031 us for forward and
+// backward, scale 18 517 -> 510.  Others lose by it (256 stacked ER graphs, k =
+// 128: 1349 -> 1365 us; 512, k = 64: 2103 -> 2142).
 // Work item wi = (column block, task, row group), the group fastest, so the
 // G warps of one tile-row read its structure at about the same time.
-template <int T, int IPW, int VEC, bool FULL, typename V>
+template <int T, int IPW, int VEC, bool FULL, bool STREAM, typename V>
 __global__ void __launch_bounds__(ROWS_WARPS * 32, ROWS_BLOCKS)
 spmm_rows_kernel(SpmmRowsArgs<V> a) {
     using P = RowsPack<T>;
@@ -333,7 +336,7 @@ spmm_rows_kernel(SpmmRowsArgs<V> a) {
             int tc = 0;
             RowsWord<T> w;
             if (more && j < t.z) {
-                tc = __ldg(a.colind + j);
+                tc = STREAM ? __ldcs(a.colind + j) : __ldg(a.colind + j);
                 w.load(a.tiles, j, gi);
             }
             // inclusive scan of the packed per-row counts of this step
@@ -468,31 +471,17 @@ spmm_rows_kernel(SpmmRowsArgs<V> a) {
             if (writer) {
 #pragma unroll
                 for (int r = 0; r < R; ++r)
-                    rows_store<V, VEC, FULL, LPI>(a.Y + ((long long)t.x * T + r0 + r) * a.ldy + col, acc[r], nvalid,
-                                                  a.accumulate != 0);
+                    rows_store<V, VEC, FULL, LPI, STREAM>(a.Y + ((long long)t.x * T + r0 + r) * a.ldy + col, acc[r], nvalid,
+                                                          a.accumulate != 0);
             }
             continue;
         }
-        // a segment of a long row: its partial rows to the slot, then count in
+        // a segment of a long row: its partial rows to the slot
         V* dst = a.partials + ((long long)t.w * T + r0) * a.k + col;
         if (writer) {
 #pragma unroll
             for (int r = 0; r < R; ++r) rows_store<V, VEC, FULL, LPI>(dst + (long long)r * a.k, acc[r], nvalid, false);
         }
-        __threadfence();
-        __syncwarp();
-        int lr = 0, last = 0;
-        if (lane == 0) {
-            lr = __ldg(a.slot_long + t.w);
-            // arrivals per (long row, row group): each segment once per column block
-            last = atomicAdd(a.state + 2 + lr * G + gi, 1) == __ldg(a.long_rows + lr).z * a.ncb - 1;
-        }
-        if (!__shfl_sync(FULL_MASK, last, 0)) continue;
-        // the group's last segment: its Y rows (+)= its slots added in segment order
-        lr = __shfl_sync(FULL_MASK, lr, 0);
-        __threadfence();
-        rows_long_reduce<T, IPW, VEC, FULL, V>(a, lr, lane, r0);
-        if (lane == 0) a.state[2 + lr * G + gi] = 0;
     }
 }
 
@@ -502,10 +491,19 @@ spmm_rows_kernel(SpmmRowsArgs<V> a) {
 // stays balanced at every graph size.  The best of 20/30/40% on R-MAT scales
 // 16-20 with k = 64 and 128 on GB300; 40% fell off a cliff at T = 4 (the
 // queue's end waits on long segments).
+// The least segments, for the hubs of small graphs, and the tile-rows that stay
+// whole whatever the share: cutting an ordinary tile-row costs more in slots
+// and the second kernel than it wins (8140 x 4798 with 29 entries a row, 194
+// tiles a tile-row at T = 8, k = 3: 21 us in two segments, 17 whole).  Segments
+// of at least 128 tiles and 1024 bits instead: R-MAT scale 12 / 14 at T = 8, k =
+// 64 46 / 58 us (31 / 28 with these), scale 14 at T = 4 43 (27), scale 16 at
+// T = 16, k = 128 186 (117).
+constexpr long long ROWS_MIN_TILES = 32, ROWS_MIN_BITS = 512;
+constexpr int ROWS_WHOLE_TILES = 256, ROWS_WHOLE_BITS = 1024;
 int spmm_rows_seg(int T, long long nt, int num_sms) {
     const long long visits = nt * (T / ROWS_R);
     const long long warps = (long long)std::max(num_sms, 1) * ROWS_BLOCKS * ROWS_WARPS;
-    return (int)std::min(8192LL, std::max(128LL, visits * 30 / (100 * warps)));
+    return (int)std::min(8192LL, std::max(ROWS_MIN_TILES, visits * 30 / (100 * warps)));
 }
 
 // Set bits of every tile-row, into zeroed bits[nb].  A warp takes 512 tiles in
@@ -576,7 +574,8 @@ b2sr_status spmm_rows_plan_create(const int* d_rowptr, const void* d_tiles, int 
     // still run together: R-MAT scale 18 / 20 as fast as longest first, and
     // 512 stacked ER graphs 1.86 ms against 2.85 ms longest first (2.61 ms in
     // row order with fixed segments).
-    PlanRule rule{T == 4 ? PlanRule::TWO : PlanRule::BITS, spmm_rows_seg(T, nt, num_sms), T == 4 ? 2 : PLAN_CLASSES};
+    PlanRule rule{T == 4 ? PlanRule::TWO : PlanRule::BITS, spmm_rows_seg(T, nt, num_sms), T == 4 ? 2 : PLAN_CLASSES,
+                  0, 0, NARROW_SLOTS, ROWS_WHOLE_TILES, ROWS_WHOLE_BITS};
     // T >= 8: segments also bounded by their set bits, at most 70% of a
     // resident warp's share of all of them, and most set bits first.  A row
     // group holding hub rows carries far more set bits than its tiles suggest
@@ -602,19 +601,16 @@ b2sr_status spmm_rows_plan_create(const int* d_rowptr, const void* d_tiles, int 
         if (nt > 0 && T == 32) tile_row_bits_kernel<32><<<blocks, 256, 0, s>>>(d_rowptr, d_tiles, nb, nt, bits);
         rule.row_bits = d_bits;
         const long long warps = (long long)std::max(num_sms, 1) * ROWS_BLOCKS * ROWS_WARPS;
-        rule.seg_bits = std::max(1024LL, nnz * 7 / (10 * warps));
+        rule.seg_bits = std::max(ROWS_MIN_BITS, nnz * 7 / (10 * warps));
     }
     const PlanBounds cap = plan_bounds(rule, nb, nt, nnz);
-    const size_t longs_at = sizeof(int4) * (size_t)cap.tasks, slots_at = longs_at + sizeof(int4) * (size_t)cap.longs;
     SpmmRowsPlan p;
-    p.groups = T / ROWS_R;
-    p.d_tasks = static_cast<int4*>(dev_alloc(slots_at + sizeof(int) * (size_t)cap.slots));
+    p.d_tasks = static_cast<int4*>(dev_alloc(sizeof(int4) * (size_t)(cap.tasks + cap.longs)));
     b2sr_status st = B2SR_ERR_ALLOC;
     PlanTotals t;
     if (p.d_tasks) {
         p.d_long = p.d_tasks + cap.tasks;
-        p.d_slot_long = reinterpret_cast<int*>(p.d_long + cap.longs);
-        st = build_plan(rule, d_rowptr, nb, cap, p.d_tasks, p.d_long, p.d_slot_long, &t, s);
+        st = build_plan(rule, d_rowptr, nb, cap, p.d_tasks, p.d_long, &t, s);
     } else {
         cudaStreamSynchronize(s);  // the set-bit count
     }
@@ -625,16 +621,16 @@ b2sr_status spmm_rows_plan_create(const int* d_rowptr, const void* d_tiles, int 
     }
     p.ntasks = t.tasks;
     p.nlong = t.longs;
+    p.nnarrow = t.narrow;
     p.nslots = t.slots;
     *out = p;
     return B2SR_SUCCESS;
 }
 
 void spmm_rows_plan_free(SpmmRowsPlan* p) {
-    dev_free(p->d_tasks);  // the others are part of it
+    dev_free(p->d_tasks);  // d_long is part of it
     p->d_tasks = nullptr;
     p->d_long = nullptr;
-    p->d_slot_long = nullptr;
 }
 
 // Columns of a warp pass (LPI * VEC) and of a lane.  rhs_block > 0 (FP32
@@ -658,13 +654,13 @@ size_t spmm_rows_scratch_bytes(const SpmmRowsPlan& p, int T, int elem_bytes, int
     return (size_t)std::max(p.nslots, 1) * T * (size_t)k * elem_bytes;
 }
 
-size_t spmm_rows_state_bytes(const SpmmRowsPlan& p) { return sizeof(int) * (2 + (size_t)p.nlong * p.groups); }
+size_t spmm_rows_state_bytes() { return 2 * sizeof(int); }
 
-template <int T, int IPW, int VEC, bool FULL, typename V>
-static b2sr_status run_rows(SpmmRowsArgs<V> a, int num_sms, cudaStream_t s) {
+template <int T, int IPW, int VEC, bool FULL, bool STREAM, typename V>
+static b2sr_status run_rows(SpmmRowsArgs<V> a, const SpmmRowsPlan& p, int num_sms, cudaStream_t s) {
     constexpr int SMEM = ROWS_WARPS * ROWS_R * ROWS_CAP * (int)sizeof(int);
     // per device: the attribute is set on every launch (cheap), the occupancy once
-    cudaError_t e = cudaFuncSetAttribute(spmm_rows_kernel<T, IPW, VEC, FULL, V>,
+    cudaError_t e = cudaFuncSetAttribute(spmm_rows_kernel<T, IPW, VEC, FULL, STREAM, V>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
     if (e != cudaSuccess) {
         set_cuda_error(e);
@@ -673,7 +669,7 @@ static b2sr_status run_rows(SpmmRowsArgs<V> a, int num_sms, cudaStream_t s) {
     static int blocks_per_sm = 0;  // per instantiation; the device's SM count scales it
     if (blocks_per_sm == 0) {
         int n = 0;
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, spmm_rows_kernel<T, IPW, VEC, FULL, V>, ROWS_WARPS * 32,
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, spmm_rows_kernel<T, IPW, VEC, FULL, STREAM, V>, ROWS_WARPS * 32,
                                                           SMEM);
         if (e != cudaSuccess) {
             set_cuda_error(e);
@@ -687,34 +683,45 @@ static b2sr_status run_rows(SpmmRowsArgs<V> a, int num_sms, cudaStream_t s) {
     // the queue counter is 32 bits and ends at nwork + one fetch per warp
     if (nwork + (long long)grid * ROWS_WARPS >= 0xffffffffLL) return B2SR_ERR_NOT_SUPPORTED;
     kernel_timer_mark(s, true);
-    spmm_rows_kernel<T, IPW, VEC, FULL, V><<<grid, ROWS_WARPS * 32, SMEM, s>>>(a);
+    spmm_rows_kernel<T, IPW, VEC, FULL, STREAM, V><<<grid, ROWS_WARPS * 32, SMEM, s>>>(a);
     kernel_timer_mark(s, false);
     B2SR_LAUNCH_CHECK();
     add_launch_count(1);
+    if (p.nlong > 0) {
+        const int fcb = (a.k + 32 * (FULL ? VEC : 1) - 1) / (32 * (FULL ? VEC : 1));
+        const long long narrow = ((long long)p.nnarrow * T * fcb + ROWS_WARPS - 1) / ROWS_WARPS;
+        const long long blocks = narrow + (long long)(p.nlong - p.nnarrow) * T * fcb;
+        if (blocks > 0x7fffffffLL) return B2SR_ERR_NOT_SUPPORTED;
+        B2SR_CUDA_TRY(launch_dependent(rows_fixup_kernel<T, FULL, V>, (unsigned)blocks, ROWS_WARPS * 32u, s, a,
+                                       p.nnarrow, (int)narrow, fcb));
+        add_launch_count(1);
+    }
     return B2SR_SUCCESS;
 }
 
 template <int T, typename V>
-static b2sr_status rows_dispatch(const SpmmRowsArgs<V>& a, RowsWidth w, bool full, int num_sms, cudaStream_t s) {
+static b2sr_status rows_dispatch(const SpmmRowsArgs<V>& a, RowsWidth w, bool full, const SpmmRowsPlan& p,
+                                 int num_sms, cudaStream_t s) {
     constexpr int MOST = 16 / (int)sizeof(V);
     if (full) {
         switch (w.ipw) {
-            case 1: return run_rows<T, 1, MOST, true, V>(a, num_sms, s);
-            case 2: return run_rows<T, 2, MOST, true, V>(a, num_sms, s);
-            case 4: return run_rows<T, 4, MOST, true, V>(a, num_sms, s);
-            default: return run_rows<T, 8, MOST, true, V>(a, num_sms, s);
+            case 1: return p.nlong > 0 ? run_rows<T, 1, MOST, true, true, V>(a, p, num_sms, s)
+                                       : run_rows<T, 1, MOST, true, false, V>(a, p, num_sms, s);
+            case 2: return run_rows<T, 2, MOST, true, false, V>(a, p, num_sms, s);
+            case 4: return run_rows<T, 4, MOST, true, false, V>(a, p, num_sms, s);
+            default: return run_rows<T, 8, MOST, true, false, V>(a, p, num_sms, s);
         }
     }
-    if (w.vec == 2) return run_rows<T, 1, 2, false, V>(a, num_sms, s);
+    if (w.vec == 2) return run_rows<T, 1, 2, false, false, V>(a, p, num_sms, s);
     if constexpr (MOST == 4) {
-        if (w.vec == 3) return run_rows<T, 1, 3, false, V>(a, num_sms, s);
-        if (w.vec == 4) return run_rows<T, 1, 4, false, V>(a, num_sms, s);
+        if (w.vec == 3) return run_rows<T, 1, 3, false, false, V>(a, p, num_sms, s);
+        if (w.vec == 4) return run_rows<T, 1, 4, false, false, V>(a, p, num_sms, s);
     }
     switch (w.ipw) {
-        case 1: return run_rows<T, 1, 1, false, V>(a, num_sms, s);
-        case 2: return run_rows<T, 2, 1, false, V>(a, num_sms, s);
-        case 4: return run_rows<T, 4, 1, false, V>(a, num_sms, s);
-        default: return run_rows<T, 8, 1, false, V>(a, num_sms, s);
+        case 1: return run_rows<T, 1, 1, false, false, V>(a, p, num_sms, s);
+        case 2: return run_rows<T, 2, 1, false, false, V>(a, p, num_sms, s);
+        case 4: return run_rows<T, 4, 1, false, false, V>(a, p, num_sms, s);
+        default: return run_rows<T, 8, 1, false, false, V>(a, p, num_sms, s);
     }
 }
 
@@ -742,13 +749,12 @@ b2sr_status spmm_rows_launch(const MatView& A, const SpmmRowsPlan& p, const V* X
     a.ntasks = p.ntasks;
     a.state = state;
     a.long_rows = p.d_long;
-    a.slot_long = p.d_slot_long;
     a.partials = static_cast<V*>(scratch);
     a.accumulate = accumulate;
-    if (A.T == 4) return rows_dispatch<4, V>(a, w, full, num_sms, s);
-    if (A.T == 8) return rows_dispatch<8, V>(a, w, full, num_sms, s);
-    if (A.T == 16) return rows_dispatch<16, V>(a, w, full, num_sms, s);
-    if (A.T == 32) return rows_dispatch<32, V>(a, w, full, num_sms, s);
+    if (A.T == 4) return rows_dispatch<4, V>(a, w, full, p, num_sms, s);
+    if (A.T == 8) return rows_dispatch<8, V>(a, w, full, p, num_sms, s);
+    if (A.T == 16) return rows_dispatch<16, V>(a, w, full, p, num_sms, s);
+    if (A.T == 32) return rows_dispatch<32, V>(a, w, full, p, num_sms, s);
     return B2SR_ERR_INVALID_VALUE;
 }
 
