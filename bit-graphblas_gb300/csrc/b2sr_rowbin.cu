@@ -734,34 +734,39 @@ __device__ __forceinline__ void bits_group(const RowBinBitsArgs& a, int task, bo
         if (KIND == 1) m &= ~(uint32_t)__ldg(static_cast<const W*>(a.mask) + t.x);
         *y = (W)(a.accumulate ? ((uint32_t)*y | m) : m);
     } else {
-        int acc[T];
+        // counts of rows 2k and 2k + 1 in the halves of acc[k]: half the
+        // registers and half the shuffles of a count per word (T = 16, R-MAT
+        // scale 20: 138.9 -> 124.9 us with the register cap that it allows;
+        // T = 8 74.5 -> 72.4, T = 4 the same)
+        constexpr int H = T / 2;
+        static_assert(G * U * T < 65536, "a task's count of a row fits 16 bits");
+        int acc[H];
 #pragma unroll
-        for (int r = 0; r < T; ++r) acc[r] = 0;
+        for (int k = 0; k < H; ++k) acc[k] = 0;
 #pragma unroll
         for (int u = 0; u < U; ++u)
             if (tc[u] >= 0) {
 #pragma unroll
-                for (int r = 0; r < T; ++r) acc[r] += __popc(bits[u].row(r) & xw[u]);
+                for (int r = 0; r < T; ++r) acc[r / 2] += __popc(bits[u].row(r) & xw[u]) << (16 * (r & 1));
             }
-        const int first = group_reduce<T, SemSumI32, G>(acc, l);
-        constexpr int NV = T >= G ? T / G : 1;
-        const bool writer = (T >= G) || ((l & (G / T - 1)) == 0);
+        const int first = group_reduce<H, SemSumI32, G>(acc, l);
+        constexpr int NV = H >= G ? H / G : 1;
+        const bool writer = (H >= G) || ((l & (G / H - 1)) == 0);
         if (!valid || !writer || t.w == -2) return;
         if (t.w >= 0) {
-            int* dst = static_cast<int*>(a.partials) + (size_t)t.w * T + first;
+            int2* dst = reinterpret_cast<int2*>(static_cast<int*>(a.partials) + (size_t)t.w * T) + first;
 #pragma unroll
-            for (int k = 0; k < NV; ++k) dst[k] = acc[k];
+            for (int k = 0; k < NV; ++k) dst[k] = make_int2(acc[k] & 0xFFFF, (int)((unsigned)acc[k] >> 16));
             return;
         }
-        const size_t off = (size_t)t.x * T + first;
-        if constexpr (KIND == 2) {
-            int* dst = static_cast<int*>(a.y) + off;
+        const size_t off = (size_t)t.x * T + 2 * first;
+        using Y = typename std::conditional<KIND == 2, int, float>::type;
+        Y* dst = static_cast<Y*>(a.y) + off;
 #pragma unroll
-            for (int k = 0; k < NV; ++k) dst[k] = a.accumulate ? dst[k] + acc[k] : acc[k];
-        } else {
-            float* dst = static_cast<float*>(a.y) + off;
-#pragma unroll
-            for (int k = 0; k < NV; ++k) dst[k] = a.accumulate ? dst[k] + (float)acc[k] : (float)acc[k];
+        for (int k = 0; k < NV; ++k) {
+            const Y lo = (Y)(acc[k] & 0xFFFF), hi = (Y)((unsigned)acc[k] >> 16);
+            dst[2 * k] = a.accumulate ? dst[2 * k] + lo : lo;
+            dst[2 * k + 1] = a.accumulate ? dst[2 * k + 1] + hi : hi;
         }
     }
 }
@@ -772,12 +777,11 @@ __device__ __forceinline__ void wide_bits_rows(const RowBinBitsArgs& a, int task
     for (int p = 0; p < 2; ++p) wide_bits_group<T, KIND, G>(a, task0 + p * (WIDE_PASS<T> / G), tend, skip);
 }
 
-// T <= 8 fits 32 registers: 64 warps per SM.  So do the T = 16 bit kernels
-// (bin_bin_bin, masked) without spills: 64 warps per SM instead of 48 at 40,
-// R-MAT scale 20 121.5 instead of 133.1 us per call (the count kinds spill at
-// such a cap).  T = 32 fits 40: 48 warps.
+// T <= 16 fits 32 registers: 64 warps per SM.  At T = 16 on R-MAT scale 20 the
+// bit kinds (no spills) take 121.5 instead of 133.1 us at 40 registers, the
+// count kinds (a few spills) 124.9 instead of 128.6.  T = 32 fits 40: 48 warps.
 template <int T, int KIND>
-__global__ void __launch_bounds__(256, T <= 8 ? 8 : 1) __maxnreg__((T == 32 ? 40 : T == 16 && KIND <= 1 ? 32 : 255))
+__global__ void __launch_bounds__(256, T <= 8 ? 8 : 1) __maxnreg__((T == 32 ? 40 : T == 16 ? 32 : 255))
     rowbin_bits_kernel(RowBinBitsArgs a) {
     const int warp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     const int lane = threadIdx.x & 31;
