@@ -9,8 +9,8 @@
 //   1. validate the CSR, an entry per thread (which also counts duplicates, so
 //      the number of set bits is known without reading the tiles);
 //   2. cut every tile-row into chunks of about 400 (T = 4) or 320 entries;
-//   3. a warp per chunk sorts the chunk's entries by (tile-column, row, column)
-//      in registers, writes the sorted keys and counts the tiles;
+//   3. a warp per chunk sorts the chunk's entries by (tile-column, row, column),
+//      by merging its rows (T <= 8) or in registers, writes the sorted keys and counts the tiles;
 //   4. scans give the tile-row pointer and the tile count (the one value the
 //      host waits for, to allocate the result);
 //   5. a warp per chunk reads its sorted keys back and assembles the tiles in
@@ -200,6 +200,63 @@ __device__ __forceinline__ void warp_sort(Key (&key)[K], int lane) {
 // e = lane*K + k and e = k*32 + lane are free of bank conflicts.
 __device__ __forceinline__ int spread(int e) { return e + (e >> 5); }
 
+// The keys of a chunk lie in buf row after row, each row's ascending, row r's
+// from pre[r] to pre[r + 1]: merges neighbouring rows, then neighbouring pairs
+// and so on, until key[k] is element lane*K + k of the whole (~0 past the end).
+// A lane makes K consecutive elements of a round; a binary search finds where
+// they begin in the two runs they come from.
+// Packing R-MAT scale 20 by merging instead of sorting: T = 4 806 -> 726 us,
+// T = 8 816 -> 768, T = 16 870 -> 878, T = 32 3018 -> 3080 (a round for every
+// doubling of T, where the sort's cost does not depend on T); for chunks of at
+// most 128 entries too: T = 4 728, T = 8 778.
+template <int T, int K> constexpr bool MERGES_ROWS = T <= 8 && K >= 8;
+template <int T, typename Key, int K>
+__device__ __forceinline__ void merge_rows(Key (&key)[K], Key* buf, const int* pre, int n, int lane) {
+    const int o = lane * K;
+#pragma unroll 1
+    for (int span = 1; span < T; span <<= 1) {
+        int r = 0;  // first row of the last pair of runs with pre <= o
+#pragma unroll 1
+        for (int step = T / 2; step >= 2 * span; step >>= 1)
+            if (pre[r + step] <= o) r += step;
+        int a = pre[r], b = pre[r + span], aend = b, bend = pre[r + 2 * span];
+        const int d = min(o, n) - a;
+        int lo = max(0, d - (bend - b)), hi = min(d, aend - a);
+        while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if (buf[spread(a + mid)] < buf[spread(b + d - 1 - mid)]) lo = mid + 1;
+            else hi = mid;
+        }
+        a += lo;
+        b += d - lo;
+        Key ka = a < aend ? buf[spread(a)] : ~Key(0), kb = b < bend ? buf[spread(b)] : ~Key(0);
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            while ((ka & kb) == ~Key(0) && r + 2 * span < T) {  // the next pair of runs
+                r += 2 * span;
+                a = bend;
+                b = aend = pre[r + span];
+                bend = pre[r + 2 * span];
+                ka = a < aend ? buf[spread(a)] : ~Key(0);
+                kb = b < bend ? buf[spread(b)] : ~Key(0);
+            }
+            const bool ta = ka < kb;
+            key[k] = ta ? ka : kb;
+            const int i = ta ? ++a : ++b;
+            const Key v = i < (ta ? aend : bend) ? buf[spread(i)] : ~Key(0);
+            if (ta) ka = v;
+            else kb = v;
+        }
+        if (2 * span < T) {
+            __syncwarp();
+#pragma unroll
+            for (int k = 0; k < K; ++k)
+                if (o + k < n) buf[spread(o + k)] = key[k];
+            __syncwarp();
+        }
+    }
+}
+
 // A chunk as its warp sees it: lane r < T holds row r's first entry in the
 // chunk, and how many entries the rows before it have there.
 struct ChunkRows {
@@ -211,7 +268,7 @@ struct ChunkRows {
 // number of distinct tile-columns.  buf: spread(32*K) keys of shared memory.
 template <int T, typename Key, int K>
 __device__ __forceinline__ int sort_chunk(const int* __restrict__ colind, const ChunkRows& c, Key* __restrict__ sorted,
-                                          Key* buf, int lane) {
+                                          Key* buf, int* pre, int lane) {
     constexpr int LT = Log2<T>::value;
     Key key[K];
     constexpr int L = K < 8 ? K : 8;  // loads in flight
@@ -234,7 +291,17 @@ __device__ __forceinline__ int sort_chunk(const int* __restrict__ colind, const 
 #pragma unroll
         for (int k = 0; k < L; ++k) key[k0 + k] = col[k] >= 0 ? pack_key<T, Key>(row[k], col[k]) : ~Key(0);
     }
-    warp_sort<Key, K>(key, lane);
+    if constexpr (MERGES_ROWS<T, K>) {
+        if (lane < T) pre[lane] = c.pre;
+        if (lane == 0) pre[T] = c.n;
+#pragma unroll
+        for (int k = 0; k < K; ++k) buf[spread(k * 32 + lane)] = key[k];
+        __syncwarp();
+        merge_rows<T, Key, K>(key, buf, pre, c.n, lane);
+        __syncwarp();
+    } else {
+        warp_sort<Key, K>(key, lane);
+    }
     Key prev = __shfl_up_sync(FULL_MASK, key[K - 1], 1);
     int tiles = 0;
 #pragma unroll
@@ -288,14 +355,17 @@ constexpr int PACK_WARPS = 8;
 
 // Step 3.  ccount[c] = tiles of chunk c (0 past the last chunk); coff_e[c] =
 // its first entry in `sorted` (chunks are in entry order; coff_e[chunks] = nnz).
-// Five blocks per SM with 32-bit keys (48 registers, 8 bytes spilled).
+// Blocks per SM with 32-bit keys, T <= 8 and above: 6 (40 registers) and 5 (48), a
+// few bytes spilled: R-MAT scale 20, T = 4, 738 us with 5 and 722 with 6, T =
+// 32 the same.
 template <int T, typename Key>
-__global__ void __launch_bounds__(PACK_WARPS * 32, sizeof(Key) == 4 ? 5 : 1)
+__global__ void __launch_bounds__(PACK_WARPS * 32, sizeof(Key) == 4 ? (T <= 8 ? 6 : 5) : 1)
 chunk_sort_kernel(const int* __restrict__ rowptr, const int* __restrict__ colind, int nrows, int nb,
                   const int* __restrict__ choff, const int* __restrict__ chunk_tr, int max_chunks,
                   int* __restrict__ ccount, int* __restrict__ coff_e, Key* __restrict__ sorted) {
     constexpr int LT = Log2<T>::value;
     __shared__ Key s_buf[PACK_WARPS][CHUNK_CAP + CHUNK_CAP / 32];
+    __shared__ int s_pre[PACK_WARPS][T + 1];
     const int lane = threadIdx.x & 31;
     const long long cl = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (cl > max_chunks) return;
@@ -352,11 +422,11 @@ chunk_sort_kernel(const int* __restrict__ rowptr, const int* __restrict__ colind
     Key* out = sorted + at;
     int tiles;
     if (rows.n > CHUNK_CAP) tiles = merge_chunk<T, Key>(colind, p, e, out, lane);
-    else if (rows.n > 256) tiles = sort_chunk<T, Key, 16>(colind, rows, out, buf, lane);
-    else if (rows.n > 128) tiles = sort_chunk<T, Key, 8>(colind, rows, out, buf, lane);
-    else if (rows.n > 64) tiles = sort_chunk<T, Key, 4>(colind, rows, out, buf, lane);
-    else if (rows.n > 32) tiles = sort_chunk<T, Key, 2>(colind, rows, out, buf, lane);
-    else tiles = sort_chunk<T, Key, 1>(colind, rows, out, buf, lane);
+    else if (rows.n > 256) tiles = sort_chunk<T, Key, 16>(colind, rows, out, buf, s_pre[threadIdx.x >> 5], lane);
+    else if (rows.n > 128) tiles = sort_chunk<T, Key, 8>(colind, rows, out, buf, s_pre[threadIdx.x >> 5], lane);
+    else if (rows.n > 64) tiles = sort_chunk<T, Key, 4>(colind, rows, out, buf, s_pre[threadIdx.x >> 5], lane);
+    else if (rows.n > 32) tiles = sort_chunk<T, Key, 2>(colind, rows, out, buf, s_pre[threadIdx.x >> 5], lane);
+    else tiles = sort_chunk<T, Key, 1>(colind, rows, out, buf, s_pre[threadIdx.x >> 5], lane);
     if (lane == 0) {
         ccount[c] = tiles;
         coff_e[c] = at;

@@ -98,3 +98,30 @@ def test_transpose_digit_passes(pkg, orc, cuda, T):
         for a, b in zip(B.transpose().download(), want):
             np.testing.assert_array_equal(a, b)
         B.close()
+
+
+@pytest.mark.parametrize("T", [4, 8])
+@pytest.mark.parametrize("ncols", [3000, 1 << 30])
+def test_rows_that_are_merged(pkg, orc, cuda, T, ncols):
+    """One tile-row per case of 129 to 512 entries: all in one row, runs of empty rows before, between
+    and behind, single entries, rows before and behind each other's columns, and equal rows."""
+    rng = np.random.default_rng(T + ncols)
+    pick = lambda n: rng.choice(min(ncols, 1 << 20), n, replace=False)  # noqa: E731
+    rows = []
+    for n in (129, 255, 256, 257, 500, 512):
+        for at in (0, 1, T - 2, T - 1):  # (others, their sizes) beside one long row
+            for rest in (0, 1):
+                tr = [pick(rest) for _ in range(T)]
+                tr[at] = pick(n - rest * (T - 1))
+                rows += tr
+        cut = np.linspace(0, n, T + 1).astype(int)
+        rows += [np.arange(cut[r], cut[r + 1]) for r in range(T)]  # ascending from row to row
+        rows += [np.arange(cut[T - 1 - r], cut[T - r]) for r in range(T)]
+        rows += [np.arange(n // T) * 5] * T
+        rows += [pick(n // 2), pick(n - n // 2)] + [[] for _ in range(T - 2)]
+        rows += [[] for _ in range(T - 2)] + [pick(n // 2), pick(n - n // 2)]
+    rowptr, colind, _ = _csr(rows, ncols)
+    A = pkg.B2SRMatrix.from_csr(rowptr, colind, len(rows), ncols, T, device=cuda)
+    for got, want in zip(A.download(), orc.csr_to_b2sr(rowptr, colind, len(rows), T)):
+        np.testing.assert_array_equal(got, want)
+    A.close()
