@@ -604,7 +604,7 @@ static b2sr_status run_rowbin(const b2sr_matrix* m_const, const float* x, float*
     st = matrix_scratch(m, s, rowbin_scratch_bytes(*plan, m->T, 4), &partials, fallback);
     if (st != B2SR_SUCCESS) return st;
     // T = 32: only set columns' x elements, whatever is asked for (whole
-    // segments: 1.04 vs 0.69 ms, R-MAT s20).  T = 16: those by default (0.28 vs
+    // segments: 1.04 vs 0.69 ms, R-MAT s20).  T = 16: those by default (0.25 vs
     // 0.34 ms).  T <= 8: whole x segments through the texture path by default
     // (measured faster there); ld.global when asked for or when x cannot back
     // a texture.

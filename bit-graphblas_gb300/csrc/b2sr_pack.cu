@@ -10,7 +10,8 @@
 //      the number of set bits is known without reading the tiles);
 //   2. cut every tile-row into chunks of about 400 (T = 4) or 320 entries;
 //   3. a warp per chunk sorts the chunk's entries by (tile-column, row, column),
-//      by merging its rows (T <= 8) or in registers, writes the sorted keys and counts the tiles;
+//      by merging its rows (T <= 8) or in registers, writes the sorted keys and
+//      counts the tiles;
 //   4. scans give the tile-row pointer and the tile count (the one value the
 //      host waits for, to allocate the result);
 //   5. a warp per chunk reads its sorted keys back and assembles the tiles in

@@ -181,14 +181,32 @@ struct SparseColTile {
     float xv[K];
     const float* xrow;  // x + tc*T
     int lim;            // columns of this tile-column inside x
+    // Bit b of row r, at T = 16 in the word of the row's pair without taking the
+    // row out of it (issue-bound: R-MAT scale 20 269.8 -> 251.6 us).  The same
+    // for T = 8 stays behind whole segments there (170 against 138 us).
+    __device__ __forceinline__ bool has(int r, uint32_t b) const {
+        if constexpr (T == 16) {
+            const uint4& v = r < 8 ? bits.a : bits.b;
+            const int k = (r & 7) >> 1;
+            const uint32_t u = k == 0 ? v.x : k == 1 ? v.y : k == 2 ? v.z : v.w;
+            return (u & ((r & 1) ? b << 16 : b)) != 0;
+        } else {
+            return (bits.row(r) & b) != 0;
+        }
+    }
     __device__ __forceinline__ void load(const W* tiles, const int* colind, int j) {
         tc = __ldcs(colind + j);
         bits.load_stream(tiles, j);
     }
     __device__ __forceinline__ void load_x(const float* __restrict__ x, int ncols, cudaTextureObject_t) {
         uint32_t cm = 0;
+        if constexpr (T == 16) {
+            const uint32_t o = bits.a.x | bits.a.y | bits.a.z | bits.a.w | bits.b.x | bits.b.y | bits.b.z | bits.b.w;
+            cm = (o | (o >> 16)) & 0xFFFFu;
+        } else {
 #pragma unroll
-        for (int r = 0; r < T; ++r) cm |= bits.row(r);
+            for (int r = 0; r < T; ++r) cm |= bits.row(r);
+        }
         const long long base = (long long)tc * T;
         xrow = x + base;
         lim = (int)(ncols - base < T ? ncols - base : T);
@@ -219,18 +237,17 @@ struct SparseColTile {
                 const float xc = c < lim ? __ldg(xrow + c) : 0.0f;
 #pragma unroll
                 for (int r = 0; r < T; ++r)
-                    if (bits.row(r) & b) acc[r] += xc;
+                    if (has(r, b)) acc[r] += xc;
                 cm &= ~b;
             }
         } else {
             float sum[T];
 #pragma unroll
             for (int r = 0; r < T; ++r) {
-                const uint32_t w = bits.row(r);
                 float s = 0.0f;
 #pragma unroll
                 for (int k = 0; k < K; ++k)
-                    if (w & cbit[k]) s += xv[k];
+                    if (has(r, cbit[k])) s += xv[k];
                 sum[r] = s;
             }
             for (uint32_t cm = rest; cm;) {
@@ -239,7 +256,7 @@ struct SparseColTile {
                 const float xc = c < lim ? __ldg(xrow + c) : 0.0f;
 #pragma unroll
                 for (int r = 0; r < T; ++r)
-                    if (bits.row(r) & b) sum[r] += xc;
+                    if (has(r, b)) sum[r] += xc;
                 cm &= ~b;
             }
 #pragma unroll
@@ -258,7 +275,8 @@ constexpr bool RB_WIDE = std::is_same<Sem, SemSumF32>::value ? (T == 32 && !SPAR
 // none; the FP32 T = 4 forms are capped through their launch bounds).  R-MAT
 // scale 20: FP32 T = 8 whole segments at 56 (36 warps per SM instead of 32 at
 // 63; 139 instead of 143 us, 48 was slower), T = 16 set columns at 64 (32
-// warps instead of 28 at 72; 264 instead of 278 us), T = 32 set columns at 80
+// warps, no spills; 56 takes 245 instead of 251 us, but ER graphs 57 instead
+// of 56), T = 32 set columns at 80
 // (24 warps instead of 20 at 86; 645 instead of 690 us).  64-frontier OR at
 // T = 4: 56 (36 warps instead of 34 at 60; R-MAT scale 18 53.5 instead of 61.4
 // us per call, 48 spilled and took 58.9).  Wide tiles: 72, and 112 with 64-bit
