@@ -215,7 +215,7 @@ typedef struct {
                              x elements of each tile's set columns (bin_full_full; the default at
                              T = 16, texture fetches at T = 4 and 8).  No effect at T = 32, nor on
                              multi-frontier products at T = 16: those always read set columns. */
-    int rhs_block;        /* dense-RHS product (bin_full_full, T = 4/8): columns per warp pass,
+    int rhs_block;        /* dense-RHS product (bin_full_full): columns per warp pass,
                              16, 32, 64 or 128 for FP32 (half for FP64); 0 = the narrowest block
                              that covers k.  Narrower blocks load more X rows per warp instruction. */
     int direction;        /* bit-vector variants (row-binned): 0 = pull over every tile-row (default),
