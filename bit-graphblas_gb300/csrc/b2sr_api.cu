@@ -556,7 +556,7 @@ static b2sr_status run_multiply(const b2sr_matrix* m, b2sr_variant v, const void
                 count.state = state + 2;
                 count.hint = hint_dev + kind;
                 count.nt = m->nt;
-                count.pct = push_percent(m->T);
+                count.pct = push_percent(m->T, kind >= 2);
                 return rowbin_bits(*plan, view_of(m), kind, x, y, mask, accumulate, scratch, PushLink{}, count, true, s);
             }
             const size_t y_bytes = kind <= 1 ? (size_t)m->nb * word_bytes(m->T) : (size_t)m->nb * m->T * 4;

@@ -347,10 +347,18 @@ b2sr_status rowbin_multi_bits(const RowBinPlan& p, const MatView& A, const void*
 // ---- direction-optimised bit-vector products (b2sr_push.cu) -------------------------
 // The push form visits only the tile-columns whose x word is non-zero, through
 // the transpose At; ctl[1] counts their tiles on the device.  Auto mode takes
-// it below push_percent(T)% of nt: the tile share at which the push kernel and
-// the row-binned pull kernel take equal time on R-MAT scale 20 (GB300; push
-// time is close to linear in that share).
-inline int push_percent(int T) { return T == 4 ? 18 : T == 8 ? 27 : T == 16 ? 45 : 85; }
+// it below push_percent(T, counts)% of nt: about the tile share at which the push
+// and the row-binned pull take equal time on R-MAT scale 20 (GB300; push time
+// is close to linear in that share).  Where that is depends on how full the
+// non-zero x words are, since a push pays an atomic per tile (bits) or per row
+// (counts) that it changes: with all bits set 6.6 / 9.6 / 27 / 41% and with one
+// bit 39 / 72 / 85+ / 41% for bits at T = 4 / 8 / 16 / 32, 9 / 12 / 12 / 8% and
+// 33 / 17 / 12 / 7% for counts; the lines lie between the two.  (One rule of
+// 18 / 27 / 45 / 85% for both kinds let counts at 30% of the tiles push in 265
+// us at T = 16 and 616 us at T = 32, where the pull takes 115 and 208.)
+inline int push_percent(int T, bool counts) {
+    return T == 4 ? 18 : T == 8 ? (counts ? 14 : 27) : T == 16 ? (counts ? 12 : 45) : (counts ? 8 : 41);
+}
 __device__ __forceinline__ bool push_chosen(const int* ctl, int mode, long long nt, int pct) {
     return mode == 2 || (long long)ctl[1] * 100 < nt * pct;
 }

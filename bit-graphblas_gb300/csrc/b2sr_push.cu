@@ -12,7 +12,7 @@
 //
 // A classify kernel lists the active tile-columns as work items of at most
 // CHUNK tiles (hub columns split across warps) and counts their tiles; in
-// auto mode the push kernel runs when that count is below push_percent(T)% of nt and
+// auto mode the push kernel runs when that count is below push_percent% of nt and
 // the pull kernels (launched after it) otherwise -- both read the count on the
 // device, so nothing waits on the host and the sequence can be captured.
 #include "b2sr_common.cuh"
@@ -231,7 +231,7 @@ b2sr_status launch_push(const MatView& At, int kind, int mode, const void* x, vo
     a.ctl = ctl;
     a.items = items;
     a.mode = mode;
-    a.pct = push_percent(At.T);
+    a.pct = push_percent(At.T, kind >= 2);
     a.nt = nt;
     a.hint = hint;
     if (link) {

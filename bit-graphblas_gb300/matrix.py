@@ -165,8 +165,8 @@ class B2SRMatrix:
         """Launch options of later multiplies of `variant`.  direction (bit-vector
         variants): "pull" visits every tile-row; "push" visits only the tile-columns
         with a non-zero x word, through the cached transpose; "auto" chooses per
-        call on the device (push when those hold under 18/27/45/85% of the tiles
-        at T = 4/8/16/32)."""
+        call on the device (push when those hold under 18/27/45/41% of the tiles
+        at T = 4/8/16/32, counts under 18/14/12/8%)."""
         cfg = _lib.LaunchConfig(threads, items_per_thread, ctas_per_sm, self.ALGORITHMS[algorithm],
                                 self.GATHERS[gather], rhs_block, self.DIRECTIONS[direction])
         _lib.check(_lib.load().b2sr_matrix_set_launch(self._h, VARIANTS[variant], C.byref(cfg)),

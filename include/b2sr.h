@@ -221,8 +221,9 @@ typedef struct {
     int direction;        /* bit-vector variants (row-binned): 0 = pull over every tile-row (default),
                              1 = auto: push through b2sr_matrix_transpose(m) when the tile-columns
                              with a non-zero x word hold under 18% (T = 4), 27% (8), 45% (16) or
-                             85% (32) of the tiles, chosen on the device per call; 2 = always push.  The transpose is built on the first
-                             such call (synchronizing), so make one before capturing a graph: during
+                             41% (32) of the tiles (counts: 18, 14, 12 or 8%), chosen on the device
+                             per call; 2 = always push.  The transpose is built on the first such
+                             call (synchronizing), so make one before capturing a graph: during
                              capture without it, auto pulls and push returns B2SR_ERR_NOT_SUPPORTED.
                              Results equal the pull's bit for bit; bin_bin_full with accumulate or
                              more than 2^24 columns always pulls.  With T < 32 the push ORs into y

@@ -35,3 +35,26 @@ def test_counts_of_full_tiles(pkg, orc, cuda, T):
         np.testing.assert_array_equal(A.spmv_bin_bin_full(xt, full.clone(), accumulate=True).cpu().numpy(),
                                       2 * want.astype(np.float32))
     A.close()
+
+
+@pytest.mark.parametrize("T,percent", [(4, 18), (8, 14), (16, 12), (32, 8), (8, 27), (16, 45), (32, 41)])
+def test_auto_direction_around_its_lines(pkg, cuda, T, percent):
+    """A band matrix, where tile-columns hold equal numbers of tiles: frontiers of a share of the
+    tile-columns just below, at and above each line, in turn, so that the next call's hint is wrong."""
+    n = 200 * T
+    rows = np.repeat(np.arange(n), 3)
+    cols = (rows + np.tile([0, 5 * T, 11 * T], n)) % n
+    A = pkg.B2SRMatrix.from_graph(pkg.from_edges(rows, cols, nrows=n, ncols=n, drop_self_loops=False), T, device=cuda)
+    dt = pkg.word_dtype(T)
+    for share in (percent - 1, percent, percent + 1, percent - 2, 100, 0, percent):
+        words = torch.zeros(A.nblockcols, dtype=torch.int64)
+        words[torch.randperm(200, generator=torch.Generator().manual_seed(share))[: 2 * share]] = 5
+        xt = words.to(dt).to(cuda)
+        got = {}
+        for d in ("pull", "auto"):
+            for v in ("bin_bin_bin", "bin_bin_count", "bin_bin_full"):
+                A.set_launch(v, direction=d)
+            got[d] = (A.spmv_bin_bin_bin(xt), A.spmv_bin_bin_count(xt), A.spmv_bin_bin_full(xt))
+        for a, b in zip(got["auto"], got["pull"]):
+            assert torch.equal(a, b), (share, T)
+    A.close()
