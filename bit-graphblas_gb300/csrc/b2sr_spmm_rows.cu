@@ -499,7 +499,13 @@ spmm_rows_kernel(SpmmRowsArgs<V> a) {
 // 64 46 / 58 us (31 / 28 with these), scale 14 at T = 4 43 (27), scale 16 at
 // T = 16, k = 128 186 (117).
 constexpr long long ROWS_MIN_TILES = 32, ROWS_MIN_BITS = 512;
-constexpr int ROWS_WHOLE_TILES = 256, ROWS_WHOLE_BITS = 1024;
+// Whole up to 256 tiles at T <= 8 and 512 above, where a tile-row of the same
+// rows has more of them, and a 4-row group takes fewer bits from each (ER, T =
+// 16, k = 128: 5678 vertices of degree 28 28.7 us with 256 tiles, 24.5 with 512;
+// 10 000 of degree 40 41.5 and 35.0; R-MAT scale 14, T = 16, k = 64 43.5 and
+// 46.6; T = 8 27.2 and 39.1).
+constexpr int rows_whole_tiles(int T) { return T <= 8 ? 256 : 512; }
+constexpr int ROWS_WHOLE_BITS = 1024;
 int spmm_rows_seg(int T, long long nt, int num_sms) {
     const long long visits = nt * (T / ROWS_R);
     const long long warps = (long long)std::max(num_sms, 1) * ROWS_BLOCKS * ROWS_WARPS;
@@ -575,7 +581,7 @@ b2sr_status spmm_rows_plan_create(const int* d_rowptr, const void* d_tiles, int 
     // 512 stacked ER graphs 1.86 ms against 2.85 ms longest first (2.61 ms in
     // row order with fixed segments).
     PlanRule rule{T == 4 ? PlanRule::TWO : PlanRule::BITS, spmm_rows_seg(T, nt, num_sms), T == 4 ? 2 : PLAN_CLASSES,
-                  0, 0, NARROW_SLOTS, ROWS_WHOLE_TILES, ROWS_WHOLE_BITS};
+                  0, 0, NARROW_SLOTS, rows_whole_tiles(T), ROWS_WHOLE_BITS};
     // T >= 8: segments also bounded by their set bits, at most 70% of a
     // resident warp's share of all of them, and most set bits first.  A row
     // group holding hub rows carries far more set bits than its tiles suggest
