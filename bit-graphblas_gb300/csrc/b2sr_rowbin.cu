@@ -742,13 +742,14 @@ struct RowOr {
             w[7] |= b.b.w & xr;
         }
     }
-    // bit T-1-r: row r is not zero
+    // bit T-1-r: row r is not zero in its T columns (at T = 4 the upper halves
+    // of the tile's and x's bytes may hold anything)
     __device__ __forceinline__ uint32_t rows() const {
         constexpr int B = T == 16 ? 16 : 8, PER = 32 / B;
         uint32_t m = 0;
 #pragma unroll
         for (int r = 0; r < T; ++r)
-            m |= (((w[r / PER] >> (B * (r % PER))) & ((1u << B) - 1)) != 0u ? 1u : 0u) << (T - 1 - r);
+            m |= (((w[r / PER] >> (B * (r % PER))) & ((1u << T) - 1)) != 0u ? 1u : 0u) << (T - 1 - r);
         return m;
     }
 };
@@ -781,7 +782,9 @@ __device__ __forceinline__ void count_rows(int (&acc)[T / 2], const TileBits<T> 
                 for (int i = 0; i < C; ++i) {
                     const int u = u0 + i;
                     if (u < U) {
-                        if constexpr (T == 4) c[i / 2] |= (b[u].w & (x[u] * 0x01010101u)) << (4 * (i & 1));
+                        // T = 4: only the lower half of the x byte, so no bit of
+                        // an unused half reaches the tile beside it
+                        if constexpr (T == 4) c[i / 2] |= (b[u].w & ((x[u] & 0xFu) * 0x01010101u)) << (4 * (i & 1));
                         else c[i] = (h ? b[u].w.y : b[u].w.x) & (x[u] * 0x01010101u);
                     }
                 }
