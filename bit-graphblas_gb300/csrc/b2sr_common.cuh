@@ -257,7 +257,7 @@ struct PlanTotals {
 };
 // Array sizes that hold the plan of a matrix with nt tiles and `bits` set bits.
 PlanBounds plan_bounds(const PlanRule& r, int nb, long long nt, long long bits);
-// Fills the arrays (of those sizes).  Synchronizes `s`.
+// Fills the arrays (of those sizes).  Synchronizes `s`, on failure too.
 b2sr_status build_plan(const PlanRule& rule, const int* rowptr, int nb, const PlanBounds& cap, int4* tasks, int4* longs,
                        PlanTotals* totals, cudaStream_t s);
 

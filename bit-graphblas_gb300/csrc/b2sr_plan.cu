@@ -188,13 +188,21 @@ b2sr_status build_plan(const PlanRule& rule, const int* rowptr, int nb, const Pl
                        PlanTotals* totals, cudaStream_t s) {
     const int nblocks = (nb + PLAN_ROWS - 1) / PLAN_ROWS;
     const long long n = (long long)(rule.classes + C_EXTRA) * nblocks;
-    if (n > INT_MAX || cap.tasks > INT_MAX || cap.slots > INT_MAX) return B2SR_ERR_OVERFLOW;
+    // every return waits for `s`: the caller frees row_bits, which kernels that
+    // it has queued may still be writing
+    if (n > INT_MAX || cap.tasks > INT_MAX || cap.slots > INT_MAX) {
+        cudaStreamSynchronize(s);
+        return B2SR_ERR_OVERFLOW;
+    }
     int* info = nullptr;
     const size_t info_ints = 128;
     static_assert(PLAN_CLASSES + C_EXTRA + 2 <= 128, "totals and the overflow flag");
     const size_t hist_bytes = (sizeof(int) * ((size_t)n + 1) + 255) / 256 * 256;
     char* scratch = static_cast<char*>(dev_alloc(sizeof(int) * info_ints + hist_bytes + exclusive_scan_scratch(n)));
-    if (!scratch) return B2SR_ERR_ALLOC;
+    if (!scratch) {
+        cudaStreamSynchronize(s);
+        return B2SR_ERR_ALLOC;
+    }
     info = reinterpret_cast<int*>(scratch);
     int* hist = reinterpret_cast<int*>(scratch + sizeof(int) * info_ints);
     int* err = info + info_ints - 1;
