@@ -363,6 +363,8 @@ b2sr_status launch_transpose(const int* rowptr, const int* colind, const void* t
     if (nt < 0 || nb < 0 || nbc < 0) return B2SR_ERR_INVALID_VALUE;
     if (nt == 0) {
         B2SR_CUDA_TRY(cudaMemsetAsync(rowptr_t, 0, sizeof(int) * ((size_t)nbc + 1), s));
+        // as below: the transpose may be used on any stream, or freed, from here on
+        B2SR_CUDA_TRY(cudaStreamSynchronize(s));
         return B2SR_SUCCESS;
     }
     if (nb == 0 || nbc == 0) return B2SR_ERR_INVALID_VALUE;  // tiles need a tile-row and a tile-column

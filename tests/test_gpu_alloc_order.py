@@ -79,3 +79,21 @@ def test_first_spmm_with_failing_allocations(pkg, cuda, T):
         A = pkg.B2SRMatrix.from_graph(g, T, device=cuda)
         assert torch.equal(A.spmm(X)[: g.nrows, 0].cpu(), torch.from_numpy(g.degrees()).float())
         A.close()
+
+
+@pytest.mark.parametrize("T", [4, 32])
+def test_transpose_of_an_empty_matrix_is_complete(pkg, cuda, T):
+    """The cached transpose may be used on any stream, and freed by the caller that lost the race to build
+    it, so its arrays are written when the call returns."""
+    A = pkg.B2SRMatrix.from_graph(pkg.from_edges([], [], nrows=500, ncols=300), T, device=cuda)
+    s = torch.cuda.Stream()
+    out = C.c_void_p()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(s):
+        queue_work()
+        rc = pkg._lib.load().b2sr_matrix_transpose(A.handle, s.cuda_stream, C.byref(out))
+        done = s.query()
+    assert rc == 0 and done
+    At = A.transpose()
+    assert (At.nrows, At.ncols, At.nblocks) == (300, 500, 0) and not At.download()[0].any()
+    A.close()
