@@ -1345,6 +1345,7 @@ b2sr_status b2sr_ref_csr2bsr_batch(const int* h_csrRowPtr, const int* h_csrColIn
         int nt = 0;
         PackJob job;
         st = job.count(d_rp, d_ci, nrows, ncols, nnz, blocksize, chk, &nt, nullptr, nullptr);
+        if (st != B2SR_SUCCESS) cudaStreamSynchronize(nullptr);  // it may have stopped before it waited
         dev_free(chk);
         if (st != B2SR_SUCCESS) break;
         if (nt != nblocks) { st = B2SR_ERR_INVALID_VALUE; break; }
