@@ -184,13 +184,16 @@ void dev_free(void* p) {
     else cudaFree(p);
 }
 
-// Waits for all work on device `dev`.
-static void sync_device(int dev) {
+// Waits for all work on device `dev`; false when that was refused (while a
+// stream is being captured it is).
+static bool sync_device(int dev) {
     int prev = dev;
     cudaGetDevice(&prev);
     if (prev != dev) cudaSetDevice(dev);
-    cudaDeviceSynchronize();
+    const bool ok = cudaDeviceSynchronize() == cudaSuccess;
+    if (!ok) cudaGetLastError();
     if (prev != dev) cudaSetDevice(prev);
+    return ok;
 }
 
 // Per-call scratch: stream-ordered pool memory unless a custom allocator is
@@ -717,6 +720,24 @@ static void free_matrix(b2sr_matrix* m) {
     delete m;
 }
 
+// Frees matrices once their device has been waited for.  Where it cannot be,
+// kernels may still read their memory, which the pool would hand out again:
+// they stay on a list that the next call takes up.
+static std::mutex g_unfreed_mu;
+static std::vector<b2sr_matrix*> g_unfreed;
+static void release_matrices(std::vector<b2sr_matrix*> drop) {
+    std::lock_guard<std::mutex> lk(g_unfreed_mu);
+    drop.insert(drop.end(), g_unfreed.begin(), g_unfreed.end());
+    g_unfreed.clear();
+    int dev = -1;
+    bool idle = false;
+    for (b2sr_matrix* m : drop) {
+        if (m->device != dev) idle = sync_device(dev = m->device);
+        if (idle) free_matrix(m);
+        else g_unfreed.push_back(m);
+    }
+}
+
 static b2sr_matrix* new_matrix(int nrows, int ncols, int T) {
     b2sr_matrix* m = new (std::nothrow) b2sr_matrix();
     if (!m) return nullptr;
@@ -800,10 +821,7 @@ static void shim_release(const void* a, const void* b, const void* c, bool all) 
             }
         }
     }
-    for (b2sr_matrix* m : drop) {
-        sync_device(m->device);
-        free_matrix(m);
-    }
+    if (!drop.empty()) release_matrices(std::move(drop));
 }
 
 }  // namespace b2sr
@@ -977,12 +995,11 @@ b2sr_status b2sr_matrix_describe(const b2sr_matrix* m, b2sr_matrix_desc* out) {
 }
 
 void b2sr_free(b2sr_matrix* m) {
-    if (!m) return;
-    sync_device(m->device);
-    free_matrix(m);
+    if (m) release_matrices({m});
 }
 
 void b2sr_trim(void) {
+    release_matrices({});
     std::lock_guard<std::mutex> lk(g_pool_mu);
     for (DevPool& p : g_pools)
         if (p.pool) {

@@ -122,6 +122,10 @@ b2sr_status b2sr_matrix_wrap(const int* d_rowptr, const int* d_colind, const voi
 b2sr_status b2sr_matrix_transpose(b2sr_matrix* m, void* stream, const b2sr_matrix** out_t);
 
 b2sr_status b2sr_matrix_describe(const b2sr_matrix* m, b2sr_matrix_desc* out);
+/* Waits for the device, then frees the matrix.  While a stream is being captured
+ * that wait is refused (and, as CUDA has it, the capture is invalidated): the
+ * memory is then given back by the next b2sr_free, b2sr_ref_release or b2sr_trim
+ * that can wait.  The handle is gone either way. */
 void b2sr_free(b2sr_matrix* m);
 
 /* Copy the B2SR arrays to host buffers sized from b2sr_matrix_describe

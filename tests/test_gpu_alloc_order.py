@@ -97,3 +97,27 @@ def test_transpose_of_an_empty_matrix_is_complete(pkg, cuda, T):
     At = A.transpose()
     assert (At.nrows, At.ncols, At.nblocks) == (300, 500, 0) and not At.download()[0].any()
     A.close()
+
+
+@pytest.mark.parametrize("later", ["free", "trim"])
+def test_free_during_a_capture_keeps_the_memory(pkg, cuda, later):
+    """The device cannot be waited for while a stream is being captured, so nothing goes back to the
+    allocator until a later call can."""
+    cu, lib = C.CDLL("libcuda.so.1"), pkg._lib.load()
+    g = pkg.erdos_renyi(2000, 8.0, seed=1)
+    s = torch.cuda.Stream()
+    with hooked(pkg) as h:
+        A, B = pkg.B2SRMatrix.from_graph(g, 8, device=cuda), pkg.B2SRMatrix.from_graph(g, 8, device=cuda)
+        A.spmm(torch.ones(g.ncols, 8, device=cuda))
+        torch.cuda.synchronize()
+        held, h.freed = len(h.blocks), 0
+        assert cu.cuStreamBeginCapture_v2(C.c_void_p(s.cuda_stream), 0) == 0
+        A.close()
+        freed, graph = h.freed, C.c_void_p()
+        cu.cuStreamEndCapture(C.c_void_p(s.cuda_stream), C.byref(graph))  # invalidated: an error, no graph
+        assert freed == 0 and len(h.blocks) == held
+        torch.cuda.synchronize()
+        B.close() if later == "free" else lib.b2sr_trim()
+        assert h.freed > 0
+        B.close()
+        assert not h.blocks
