@@ -462,7 +462,9 @@ __global__ void __launch_bounds__(256, (T == 4 && sizeof(typename Sem::V) == 4) 
 // FIX_G lanes each (32 / FIX_G rows per warp, one slot per lane); the others a
 // warp each, lane k folding slots k, k + 32, ... in order.  A group then
 // combines its lane partials with the main kernel's butterfly, so the order is
-// fixed for each row.
+// fixed for each row.  The kernel may start while the main kernel still writes
+// the partials (it waits for it), so they are read by ordinary loads, not through
+// the read-only path.
 constexpr int FIX_G = 8;
 
 __host__ __device__ __forceinline__ int fixup_warps(int nlong, int nshort) {
@@ -471,10 +473,11 @@ __host__ __device__ __forceinline__ int fixup_warps(int nlong, int nshort) {
 
 template <int T, class Sem, int G>
 __device__ __forceinline__ void fixup_group(const int4* __restrict__ long_rows, int idx, bool valid, int l,
-                                            const typename Sem::V* __restrict__ partials, typename Sem::V* y,
+                                            const typename Sem::V* partials, typename Sem::V* y,
                                             const typename Sem::V* __restrict__ mask, int accumulate) {
     using V = typename Sem::V;
     const int4 L = valid ? __ldg(long_rows + idx) : make_int4(0, 0, 0, 0);
+    griddep_wait();  // launched behind the main kernel: its partials
     V acc[T];
 #pragma unroll
     for (int r = 0; r < T; ++r) acc[r] = Sem::zero();
@@ -489,7 +492,7 @@ __device__ __forceinline__ void fixup_group(const int4* __restrict__ long_rows, 
             if (k < L.z) {
                 const uint4* p = reinterpret_cast<const uint4*>(partials + (size_t)(L.y + k) * T);
 #pragma unroll
-                for (int q = 0; q < (int)(T * sizeof(V) / 16); ++q) reinterpret_cast<uint4*>(v[u])[q] = __ldg(p + q);
+                for (int q = 0; q < (int)(T * sizeof(V) / 16); ++q) reinterpret_cast<uint4*>(v[u])[q] = p[q];
             }
         }
 #pragma unroll
@@ -514,9 +517,8 @@ __device__ __forceinline__ void fixup_group(const int4* __restrict__ long_rows, 
 template <int T, class Sem>
 __global__ void __launch_bounds__(256)
 rowbin_fixup_kernel(const int4* __restrict__ long_rows, int nlong, int nshort,
-                    const typename Sem::V* __restrict__ partials, typename Sem::V* __restrict__ y,
+                    const typename Sem::V* partials, typename Sem::V* __restrict__ y,
                     const typename Sem::V* __restrict__ mask, int accumulate) {
-    griddep_wait();  // launched behind the main kernel: its partials
     const int w = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     const int lane = threadIdx.x & 31;
     const int short_warps = (nshort + 32 / FIX_G - 1) / (32 / FIX_G);
@@ -934,15 +936,17 @@ __global__ void __launch_bounds__(256, T <= 8 ? 8 : 1) __maxnreg__((T == 32 ? 40
 }
 
 // Long rows: combine the segment slots (OR of words, or exact int sums), with
-// the lane groups of rowbin_fixup_kernel.
+// the lane groups and loads of rowbin_fixup_kernel.
 template <int T, int KIND, int G>
 __device__ __forceinline__ void bits_fixup_group(const RowBinBitsArgs& a, const int4* __restrict__ long_rows, int idx,
                                                  bool valid, int l) {
     using W = typename TileWord<T>::type;
     const int4 L = valid ? __ldg(long_rows + idx) : make_int4(0, 0, 0, 0);
+    griddep_wait();  // launched behind the main kernel: its partials
+    if (pull_skipped(a)) return;
     if constexpr (KIND <= 1) {
         uint32_t m = 0;
-        for (int k = l; k < L.z; k += G) m |= __ldg(static_cast<const uint32_t*>(a.partials) + L.y + k);
+        for (int k = l; k < L.z; k += G) m |= static_cast<const uint32_t*>(a.partials)[L.y + k];
 #pragma unroll
         for (int sh = G / 2; sh >= 1; sh >>= 1) m |= __shfl_xor_sync(FULL_MASK, m, sh);
         if (!valid || l != 0) return;
@@ -958,7 +962,7 @@ __device__ __forceinline__ void bits_fixup_group(const RowBinBitsArgs& a, const 
             const int4* p = reinterpret_cast<const int4*>(part + (size_t)(L.y + k) * T);
 #pragma unroll
             for (int q = 0; q < T / 4; ++q) {
-                const int4 v = __ldg(p + q);
+                const int4 v = p[q];
                 acc[4 * q] += v.x;
                 acc[4 * q + 1] += v.y;
                 acc[4 * q + 2] += v.z;
@@ -985,8 +989,6 @@ __device__ __forceinline__ void bits_fixup_group(const RowBinBitsArgs& a, const 
 template <int T, int KIND>
 __global__ void __launch_bounds__(256) rowbin_bits_fixup_kernel(RowBinBitsArgs a, const int4* __restrict__ long_rows,
                                                                 int nlong, int nshort) {
-    griddep_wait();  // launched behind the main kernel: its partials
-    if (pull_skipped(a)) return;
     const int w = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     const int lane = threadIdx.x & 31;
     const int short_warps = (nshort + 32 / FIX_G - 1) / (32 / FIX_G);

@@ -48,18 +48,23 @@ template <> struct RowsVec<double, 2> { using type = double2; };
 // A lane's VEC columns of an X or Y row.  FULL: neighbouring columns, one
 // vector load (all VEC valid and aligned).  Otherwise columns STR apart (STR
 // lanes share the row), a coalesced scalar load each, the first nvalid of them
-// inside the row: widths and strides that are no multiple of 16 bytes.
-template <typename V, int VEC, bool FULL, int STR>
+// inside the row: widths and strides that are no multiple of 16 bytes.  SLOTS:
+// rows that the launch before this one wrote, by ordinary loads: that launch may
+// still run when this kernel starts, and the read-only path (and any load that
+// the compiler need not keep behind the wait) is for data that does not change
+// while the kernel runs.
+template <typename V, int VEC, bool FULL, int STR, bool SLOTS = false>
 __device__ __forceinline__ void rows_load(V (&out)[VEC], const V* p, int nvalid) {
     if constexpr (FULL) {
         using VT = typename RowsVec<V, VEC>::type;
-        const VT v = __ldg(reinterpret_cast<const VT*>(p));
+        const VT* q = reinterpret_cast<const VT*>(p);
+        const VT v = SLOTS ? *q : __ldg(q);
         const V* e = reinterpret_cast<const V*>(&v);
 #pragma unroll
         for (int i = 0; i < VEC; ++i) out[i] = e[i];
     } else {
 #pragma unroll
-        for (int i = 0; i < VEC; ++i) out[i] = i < nvalid ? __ldg(p + i * STR) : V(0);
+        for (int i = 0; i < VEC; ++i) out[i] = i < nvalid ? (SLOTS ? p[i * STR] : __ldg(p + i * STR)) : V(0);
     }
 }
 
@@ -241,14 +246,14 @@ rows_fixup_kernel(SpmmRowsArgs<V> a, int nnarrow, int narrow_blocks, int ncb) {
         for (; q + SL <= end; q += SL) {
             V v[SL][VEC];
 #pragma unroll
-            for (int u = 0; u < SL; ++u) rows_load<V, VEC, FULL, 32>(v[u], src + (q + u) * stride, nvalid);
+            for (int u = 0; u < SL; ++u) rows_load<V, VEC, FULL, 32, true>(v[u], src + (q + u) * stride, nvalid);
 #pragma unroll
             for (int u = 0; u < SL; ++u) rows_add<V, VEC>(tot, v[u]);
         }
         if (q < end) {  // the rest, also in flight together
             V v[SL][VEC];
 #pragma unroll
-            for (int u = 0; u < SL; ++u) rows_load<V, VEC, FULL, 32>(v[u], src + (min(q + u, end - 1)) * stride, nvalid);
+            for (int u = 0; u < SL; ++u) rows_load<V, VEC, FULL, 32, true>(v[u], src + (min(q + u, end - 1)) * stride, nvalid);
 #pragma unroll
             for (int u = 0; u < SL; ++u)
                 if (q + u < end) rows_add<V, VEC>(tot, v[u]);
