@@ -59,11 +59,13 @@ validate_rows_kernel(const int* __restrict__ rowptr, int nrows, int nnz, uint32_
 // entries equal to the one before.  Four consecutive entries per thread, as one
 // 16-byte load where ALIGNED.  (A warp per row, the rows' own bounds: 357 us
 // for R-MAT scale 20; a lookup in rowptr for every entry not above the one
-// before: 112 us, issue-bound.)
+// before: 112 us, issue-bound.)  Only behind a good rowptr: with rowptr[nrows] !=
+// nnz the array may be shorter than nnz.
 template <bool ALIGNED>
 __global__ void __launch_bounds__(256)
 validate_entries_kernel(const int* __restrict__ colind, int ncols, int nnz, const uint32_t* __restrict__ starts,
                         PackInfo* __restrict__ info) {
+    if (info->flag & CSR_BAD_ROWPTR) return;  // set by validate_rows_kernel only, so uniform
     const long long p = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * 4;
     const int n = (int)(nnz - p < 4 ? nnz - p : 4);  // <= 0 past the end
     int c[4] = {0, 0, 0, 0};
