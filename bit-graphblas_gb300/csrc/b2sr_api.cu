@@ -617,6 +617,44 @@ static b2sr_status run_rowbin(const b2sr_matrix* m_const, const float* x, float*
     return rowbin_spmv(*plan, view_of(m), x, y, accumulate, partials, xtex, sparse, s);
 }
 
+static b2sr_status count_set_bits(const b2sr_matrix* m, long long* bits, cudaStream_t s) {
+    unsigned long long* d_cnt = static_cast<unsigned long long*>(dev_alloc(sizeof(unsigned long long)));
+    if (!d_cnt) return B2SR_ERR_ALLOC;
+    b2sr_status st = launch_count_bits(m->tiles, (long long)m->nt * m->T, m->T, d_cnt, s);
+    unsigned long long h = 0;
+    if (st == B2SR_SUCCESS) {
+        cudaError_t e = cudaMemcpyAsync(&h, d_cnt, sizeof(h), cudaMemcpyDeviceToHost, s);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+        if (e != cudaSuccess) {
+            set_cuda_error(e);
+            st = B2SR_ERR_CUDA;
+        }
+    }
+    if (st != B2SR_SUCCESS) cudaStreamSynchronize(s);
+    dev_free(d_cnt);
+    *bits = (long long)h;
+    return st;
+}
+
+// The row-task SpMM plan of `m`, built on first use (in a capture: as
+// ensure_rowbin).  Its arrays are sized by the set bits; the tiles of a wrapped
+// matrix may have been filled since those were counted, so where the plan does
+// not fit them they are counted again.
+static b2sr_status ensure_spmm_rows(b2sr_matrix* m, cudaStream_t s) {
+    std::lock_guard<std::mutex> lk(g_plan_mu);
+    if (m->spmm_rows_ready) return B2SR_SUCCESS;
+    if (stream_capturing(s)) return B2SR_ERR_NOT_SUPPORTED;
+    b2sr_status st = spmm_rows_plan_create(m->rowptr, m->tiles, m->nb, m->nt, m->nnz, m->T, m->num_sms, &m->spmm_rows, s);
+    if (st == B2SR_ERR_INVALID_VALUE) {
+        long long bits = 0;
+        st = count_set_bits(m, &bits, s);
+        if (st == B2SR_SUCCESS)
+            st = spmm_rows_plan_create(m->rowptr, m->tiles, m->nb, m->nt, bits, m->T, m->num_sms, &m->spmm_rows, s);
+    }
+    m->spmm_rows_ready = st == B2SR_SUCCESS;
+    return st;
+}
+
 // Chunk starts of the SpMM work queue, built on first use.
 static b2sr_status get_spmm_plan(const b2sr_matrix* m_const, cudaStream_t s, const LaunchPlan** out) {
     b2sr_matrix* m = const_cast<b2sr_matrix*>(m_const);
@@ -656,18 +694,9 @@ static b2sr_status run_spmm_api(const b2sr_matrix* m, const V* X, int k, long lo
     // row tasks with item lists, unless the bin_full_full launch option asks
     // for the merge path
     if (m->shapes[B2SR_BIN_FULL_FULL].algorithm != 1) {
-        b2sr_matrix* mm = const_cast<b2sr_matrix*>(m);
-        {
-            std::lock_guard<std::mutex> lk(g_plan_mu);
-            if (!mm->spmm_rows_ready) {
-                if (stream_capturing(s)) return B2SR_ERR_NOT_SUPPORTED;  // as ensure_rowbin
-                b2sr_status st = spmm_rows_plan_create(mm->rowptr, mm->tiles, mm->nb, mm->nt, mm->nnz, mm->T, mm->num_sms,
-                                                       &mm->spmm_rows, s);
-                if (st != B2SR_SUCCESS) return st;
-                mm->spmm_rows_ready = true;
-            }
-        }
-        b2sr_status st = matrix_scratch(m, s, spmm_rows_scratch_bytes(m->spmm_rows, m->T, (int)sizeof(V), k),
+        b2sr_status st = ensure_spmm_rows(const_cast<b2sr_matrix*>(m), s);
+        if (st != B2SR_SUCCESS) return st;
+        st = matrix_scratch(m, s, spmm_rows_scratch_bytes(m->spmm_rows, m->T, (int)sizeof(V), k),
                                         &scratch, fallback);
         if (st != B2SR_SUCCESS) return st;
         void* state = nullptr;
@@ -756,25 +785,6 @@ static b2sr_matrix* new_matrix(int nrows, int ncols, int T) {
 
 // Pads an element count so vector loads of the array tail stay inside it.
 static size_t padded_bytes(size_t bytes) { return (bytes + 255) / 256 * 256 + 256; }
-
-static b2sr_status count_set_bits(b2sr_matrix* m, cudaStream_t s) {
-    unsigned long long* d_cnt = static_cast<unsigned long long*>(dev_alloc(sizeof(unsigned long long)));
-    if (!d_cnt) return B2SR_ERR_ALLOC;
-    b2sr_status st = launch_count_bits(m->tiles, (long long)m->nt * m->T, m->T, d_cnt, s);
-    unsigned long long h = 0;
-    if (st == B2SR_SUCCESS) {
-        cudaError_t e = cudaMemcpyAsync(&h, d_cnt, sizeof(h), cudaMemcpyDeviceToHost, s);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-        if (e != cudaSuccess) {
-            set_cuda_error(e);
-            st = B2SR_ERR_CUDA;
-        }
-    }
-    if (st != B2SR_SUCCESS) cudaStreamSynchronize(s);
-    dev_free(d_cnt);
-    m->nnz = (long long)h;
-    return st;
-}
 
 // The shims' fast path.  A kernel-launch shim gets raw B2SR arrays on every
 // call, the way the reference drivers launch bmv{T}_* in their timed loops
@@ -969,7 +979,7 @@ b2sr_status b2sr_matrix_wrap(const int* d_rowptr, const int* d_colind, const voi
         return B2SR_ERR_INVALID_VALUE;
     }
     m->nt = nblocks;
-    b2sr_status st = count_set_bits(m, s);
+    b2sr_status st = count_set_bits(m, &m->nnz, s);
     if (st != B2SR_SUCCESS) {
         free_matrix(m);
         return st;
@@ -1139,7 +1149,7 @@ b2sr_status b2sr_matrix_load(const char* path, void* stream, b2sr_matrix** out) 
             st = B2SR_ERR_CUDA;
         }
     }
-    if (st == B2SR_SUCCESS) st = count_set_bits(m, s);
+    if (st == B2SR_SUCCESS) st = count_set_bits(m, &m->nnz, s);
     if (st == B2SR_SUCCESS && m->nnz != h.nnz) st = B2SR_ERR_IO;
     if (st != B2SR_SUCCESS) {
         cudaStreamSynchronize(s);
