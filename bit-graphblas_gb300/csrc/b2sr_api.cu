@@ -528,6 +528,7 @@ static b2sr_status run_multiply(const b2sr_matrix* m, b2sr_variant v, const void
         const size_t pull_bytes = dir == 2 ? 0 : (rowbin_bits_scratch_bytes(*plan, m->T) + 255) / 256 * 256;
         void* scratch = nullptr;
         Scratch fallback;
+        std::lock_guard<std::mutex> launching(mm->launch_mu);
         st = matrix_scratch(m, s, pull_bytes + (dir ? push_scratch_bytes(m->nbc, m->nt) : 0), &scratch, fallback);
         if (st != B2SR_SUCCESS) return st;
         PushLink link;
@@ -583,6 +584,7 @@ static b2sr_status run_multiply(const b2sr_matrix* m, b2sr_variant v, const void
     if (st != B2SR_SUCCESS) return st;
     void* carries = nullptr;
     Scratch fallback;
+    std::lock_guard<std::mutex> launching(const_cast<b2sr_matrix*>(m)->launch_mu);
     st = matrix_scratch(m, s, carry_bytes(v, m->T, plan->grid), &carries, fallback);
     if (st != B2SR_SUCCESS) return st;
     return launch_spmv(v, view_of(m), plan->shape, plan->grid, plan->d_starts, x, y, mask,
@@ -604,6 +606,7 @@ static b2sr_status run_rowbin(const b2sr_matrix* m_const, const float* x, float*
     if (st != B2SR_SUCCESS) return st;
     void* partials = nullptr;
     Scratch fallback;
+    std::lock_guard<std::mutex> launching(m->launch_mu);
     st = matrix_scratch(m, s, rowbin_scratch_bytes(*plan, m->T, 4), &partials, fallback);
     if (st != B2SR_SUCCESS) return st;
     // T = 32: only set columns' x elements, whatever is asked for (whole
@@ -694,8 +697,10 @@ static b2sr_status run_spmm_api(const b2sr_matrix* m, const V* X, int k, long lo
     // row tasks with item lists, unless the bin_full_full launch option asks
     // for the merge path
     if (m->shapes[B2SR_BIN_FULL_FULL].algorithm != 1) {
-        b2sr_status st = ensure_spmm_rows(const_cast<b2sr_matrix*>(m), s);
+        b2sr_matrix* mm = const_cast<b2sr_matrix*>(m);
+        b2sr_status st = ensure_spmm_rows(mm, s);
         if (st != B2SR_SUCCESS) return st;
+        std::lock_guard<std::mutex> launching(mm->launch_mu);
         st = matrix_scratch(m, s, spmm_rows_scratch_bytes(m->spmm_rows, m->T, (int)sizeof(V), k),
                                         &scratch, fallback);
         if (st != B2SR_SUCCESS) return st;
@@ -710,6 +715,7 @@ static b2sr_status run_spmm_api(const b2sr_matrix* m, const V* X, int k, long lo
     const LaunchPlan* plan = nullptr;
     b2sr_status st = get_spmm_plan(m, s, &plan);
     if (st != B2SR_SUCCESS) return st;
+    std::lock_guard<std::mutex> launching(const_cast<b2sr_matrix*>(m)->launch_mu);
     st = matrix_scratch(m, s, spmm_scratch_bytes(m->T, (int)sizeof(V), plan->grid, k), &scratch, fallback);
     if (st != B2SR_SUCCESS) return st;
     return spmm_launch<V>(view_of(m), X, ldx, Y, ldy, k, accumulate, plan->d_starts, plan->grid,
@@ -1268,6 +1274,7 @@ b2sr_status b2sr_spmv_multi_bits(const b2sr_matrix* m_const, const void* d_x, vo
     if (st != B2SR_SUCCESS) return st;
     void* partials = nullptr;
     Scratch fallback;
+    std::lock_guard<std::mutex> launching(m->launch_mu);
     st = matrix_scratch(m, s, rowbin_scratch_bytes(*plan, m->T, word_bits / 8), &partials, fallback);
     if (st != B2SR_SUCCESS) return st;
     // T >= 16 reads only set columns' words

@@ -103,6 +103,9 @@ struct b2sr_matrix {
     bool rowbin_bits_ready = false;
     b2sr::SpmmRowsPlan spmm_rows;  // row-task SpMM plan (T = 4, 8)
     bool spmm_rows_ready = false;
+    // Held while a call launches its kernels: they share the stream's scratch, so
+    // those of two host threads on one stream must not come in between.
+    std::mutex launch_mu;
     // Per-stream scratch (carries, partials, queue counter), grown on demand
     // and reused: calls on one stream are ordered, so they can share it.
     struct StreamScratch {
