@@ -208,8 +208,9 @@ private:
 // In-place exclusive scan of d_vals[0..n) with the total written to d_vals[n]
 // (d_vals has n + 1 entries), asynchronous; scratch of exclusive_scan_scratch(n)
 // bytes.  *d_err is set to 1 if the total overflows int32, else left alone.
+// Returns the kernels that it launched.
 size_t exclusive_scan_scratch(long long n);
-void exclusive_scan_async(int* d_vals, int n, int* d_err, void* scratch, cudaStream_t s);
+int exclusive_scan_async(int* d_vals, int n, int* d_err, void* scratch, cudaStream_t s);
 b2sr_status launch_pack_vec_bits(const float* x, int n, int T, void* bits, cudaStream_t s);
 b2sr_status launch_unpack_vec_bits(const void* bits, int n, int T, float* out, cudaStream_t s);
 // Set bits of a B2SR matrix (for the descriptor); result in *d_count (int64).

@@ -648,7 +648,7 @@ size_t exclusive_scan_scratch(long long n) {
     return sizeof(long long) * (size_t)((n > 0 ? (n + SCAN_TILE - 1) / SCAN_TILE : 1) + 1);
 }
 
-void exclusive_scan_async(int* vals, int n, int* err, void* scratch, cudaStream_t s) {
+int exclusive_scan_async(int* vals, int n, int* err, void* scratch, cudaStream_t s) {
     const int nblocks = n > 0 ? (n + SCAN_TILE - 1) / SCAN_TILE : 1;
     long long* partial = static_cast<long long*>(scratch);
     // one launch up to SCAN_TILE values, two while a block can add up the sums
@@ -660,6 +660,7 @@ void exclusive_scan_async(int* vals, int n, int* err, void* scratch, cudaStream_
     } else {
         scan_apply_kernel<true><<<nblocks, SCAN_THREADS, 0, s>>>(vals, n, partial, nblocks, err);
     }
+    return nblocks > SCAN_THREADS ? 3 : nblocks > 1 ? 2 : 1;
 }
 
 // ---- host side --------------------------------------------------------------------

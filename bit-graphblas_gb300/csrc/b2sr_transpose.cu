@@ -321,7 +321,7 @@ b2sr_status run_transpose(const int* rowptr, const int* colind, const void* tile
         const bool last = p + 1 == passes;
         radix_count_kernel<<<nblocks, TR_THREADS, 0, s>>>(keys, nt, shift, mask, nblocks, hist, nbc,
                                                           p == 0 ? flags + 1 : nullptr);
-        exclusive_scan_async(hist, (int)nhist, flags, mem + o_scan, s);
+        const int scans = exclusive_scan_async(hist, (int)nhist, flags, mem + o_scan, s);
         int* rows_out = last ? colind_t : row[to];
         void* load_out = last && T <= 8 ? tiles_t : load[to];
         e = p == 0 ? launch_scatter<T, true>(keys, rows, in, nt, shift, mask, nblocks, hist, key[to], rows_out, load_out, s)
@@ -329,7 +329,7 @@ b2sr_status run_transpose(const int* rowptr, const int* colind, const void* tile
         keys = key[to];
         rows = rows_out;
         in = order = load_out;
-        add_launch_count(5);
+        add_launch_count(2 + scans);
     }
     if (e == cudaSuccess) {
         transpose_rowptr_kernel<<<(unsigned)(((long long)nbc + 1 + 255) / 256), 256, 0, s>>>(keys, nt, nbc, rowptr_t);
