@@ -4,6 +4,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <deque>
 #include <mutex>
 #include <new>
 #include <unordered_map>
@@ -47,29 +48,44 @@ static b2sr_free_fn g_free = nullptr;
 static void* g_alloc_ctx = nullptr;
 
 // ---- device memory ---------------------------------------------------------------
-// Without a caller's allocator, device memory comes from one memory pool per
-// device that keeps up to 1/256 of the device's memory (1.1 GB on GB300) beyond
-// what is in use when it is freed; more goes back to the driver at the next synchronization, and all of
-// it on b2sr_trim and before an allocation fails.  cudaMalloc takes 40 - 80 us
-// and cudaFree 30 - 110 us on GB300; packing a graph, transposing it and
-// building its plans makes some 50 such calls.
+// Without a caller's allocator, device memory comes from two places per device.
+// Each keeps up to 1/512 of the device's memory (0.55 GB on GB300) that was
+// freed; all of it goes back on b2sr_trim and before an allocation fails.
+// cudaMalloc takes 40 - 80 us and cudaFree 30 - 110 us on GB300; packing a graph,
+// transposing it and building its plans makes some 50 such calls.
+//
+// Scratch, plans and counters come from a memory pool (what it holds beyond the
+// above goes back to the driver at the next synchronization).  A matrix's arrays,
+// which b2sr_matrix_describe hands out, are blocks of cudaMalloc, so that they can
+// be opened by another process (cudaIpcGetMemHandle) or another device
+// (cudaDeviceEnablePeerAccess): pool memory cannot.  Freed ones are kept whole, up
+// to 1024 of them, the oldest given up first, and taken again for sizes at most a
+// quarter smaller.
 //
 // A block is freed only when no kernel can still use it (every caller
-// synchronizes first; cudaFree used to), and all blocks are allocated and freed
-// in the order of the pool's own stream, which runs nothing else: so a block may
-// go to any stream and thread, as cudaMalloc's.
+// synchronizes first; cudaFree used to), and all blocks of the pool are allocated
+// and freed in the order of its own stream, which runs nothing else: so a block
+// may go to any stream and thread, as cudaMalloc's.
 namespace {
 struct DevPool {
     cudaMemPool_t pool = nullptr;
     cudaStream_t stream = nullptr;
     bool tried = false;
     uint64_t keep = 0, live = 0;  // bytes to keep beyond those in use; bytes in use
+    struct Kept {
+        void* ptr;
+        size_t bytes;
+    };
+    std::deque<Kept> arrays;  // freed arrays, the oldest first
+    uint64_t array_bytes = 0;
 };
 struct PoolBlock {
     DevPool* pool;
     size_t bytes;
+    bool array;  // a block of cudaMalloc
 };
 constexpr int MAX_POOLS = 64;
+constexpr size_t MAX_KEPT_ARRAYS = 1024;  // looked through by array_take
 std::mutex g_pool_mu;
 DevPool g_pools[MAX_POOLS];
 std::unordered_map<void*, PoolBlock> g_pool_blocks;  // live blocks of the pools
@@ -100,7 +116,7 @@ DevPool* device_pool(int dev) {
                   cudaStreamCreateWithFlags(&p.stream, cudaStreamNonBlocking) == cudaSuccess &&
                   cudaMemPoolCreate(&p.pool, &props) == cudaSuccess;
         if (ok) {
-            p.keep = prop.totalGlobalMem / 256;
+            p.keep = prop.totalGlobalMem / 512;
             ok = pool_use(&p, 0) == cudaSuccess;
         }
         if (!ok) {
@@ -114,19 +130,86 @@ DevPool* device_pool(int dev) {
     return p.pool ? &p : nullptr;
 }
 
+// Gives back all that is kept.
+void pool_trim(DevPool* pool) {
+    std::deque<DevPool::Kept> drop;
+    {
+        std::lock_guard<std::mutex> lk(g_pool_mu);
+        drop.swap(pool->arrays);
+        pool->array_bytes = 0;
+    }
+    for (const DevPool::Kept& k : drop) cudaFree(k.ptr);
+    cudaStreamSynchronize(pool->stream);
+    cudaMemPoolTrimTo(pool->pool, 0);
+}
+
 cudaError_t pool_alloc(DevPool* pool, void** p, size_t bytes) {
     cudaError_t e = cudaMallocFromPoolAsync(p, bytes, pool->pool, pool->stream);
     if (e == cudaErrorMemoryAllocation) {
         cudaGetLastError();
-        cudaStreamSynchronize(pool->stream);
-        cudaMemPoolTrimTo(pool->pool, 0);
+        pool_trim(pool);
         e = cudaMallocFromPoolAsync(p, bytes, pool->pool, pool->stream);
     }
     return e == cudaSuccess ? cudaStreamSynchronize(pool->stream) : e;
 }
-}  // namespace
 
-void* dev_alloc(size_t bytes) {
+// cudaMalloc also while another thread captures a stream, as the pool.
+cudaError_t malloc_relaxed(void** p, size_t bytes) {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    const cudaError_t e = cudaMalloc(p, bytes);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    return e;
+}
+
+// An array of at least *bytes; *bytes becomes its size: rounded up to an eighth
+// of a power of two where it may be kept, so that arrays of about the same size
+// (a graph per step) take each other's blocks.
+cudaError_t array_take(DevPool* pool, void** p, size_t* bytes) {
+    if (*bytes <= pool->keep) {
+        size_t step = 512;
+        while (step * 16 <= *bytes) step *= 2;
+        *bytes = (*bytes + step - 1) / step * step;
+        std::lock_guard<std::mutex> lk(g_pool_mu);
+        auto best = pool->arrays.end();
+        for (auto it = pool->arrays.begin(); it != pool->arrays.end(); ++it)
+            if (it->bytes >= *bytes && it->bytes - *bytes <= *bytes / 3 &&
+                (best == pool->arrays.end() || it->bytes < best->bytes))
+                best = it;
+        if (best != pool->arrays.end()) {
+            *p = best->ptr;
+            *bytes = best->bytes;
+            pool->array_bytes -= best->bytes;
+            pool->arrays.erase(best);
+            return cudaSuccess;
+        }
+    }
+    cudaError_t e = malloc_relaxed(p, *bytes);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        pool_trim(pool);
+        e = malloc_relaxed(p, *bytes);
+    }
+    return e;
+}
+
+// Keeps a freed array, with the oldest ones making room; what has to go to the
+// driver is appended to *drop.  With g_pool_mu held.
+void array_keep(DevPool* pool, void* p, size_t bytes, std::vector<void*>* drop) {
+    if (bytes > pool->keep) {
+        drop->push_back(p);
+        return;
+    }
+    while (pool->array_bytes + bytes > pool->keep || pool->arrays.size() >= MAX_KEPT_ARRAYS) {
+        drop->push_back(pool->arrays.front().ptr);
+        pool->array_bytes -= pool->arrays.front().bytes;
+        pool->arrays.pop_front();
+    }
+    pool->arrays.push_back({p, bytes});
+    pool->array_bytes += bytes;
+}
+
+void* alloc_block(size_t bytes, bool array) {
     if (bytes == 0) bytes = 16;
     b2sr_alloc_fn fn;
     void* ctx;
@@ -141,11 +224,11 @@ void* dev_alloc(size_t bytes) {
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) {
         DevPool* pool = device_pool(dev);
-        e = pool ? pool_alloc(pool, &p, bytes) : cudaMalloc(&p, bytes);
+        e = !pool ? cudaMalloc(&p, bytes) : array ? array_take(pool, &p, &bytes) : pool_alloc(pool, &p, bytes);
         if (pool && e == cudaSuccess) {
             std::lock_guard<std::mutex> lk(g_pool_mu);
-            g_pool_blocks[p] = {pool, bytes};
-            pool_use(pool, pool->live + bytes);
+            g_pool_blocks[p] = {pool, bytes, array};
+            if (!array) pool_use(pool, pool->live + bytes);
         }
     }
     if (e != cudaSuccess) {
@@ -155,6 +238,11 @@ void* dev_alloc(size_t bytes) {
     }
     return p;
 }
+
+}  // namespace
+
+void* dev_alloc(size_t bytes) { return alloc_block(bytes, false); }
+void* array_alloc(size_t bytes) { return alloc_block(bytes, true); }
 
 // No kernel may be using the block any more.
 void dev_free(void* p) {
@@ -171,17 +259,25 @@ void dev_free(void* p) {
         return;
     }
     DevPool* pool = nullptr;
+    std::vector<void*> drop;
     {
         std::lock_guard<std::mutex> lk(g_pool_mu);
         auto it = g_pool_blocks.find(p);
-        if (it != g_pool_blocks.end()) {
-            pool = it->second.pool;
-            pool_use(pool, pool->live - it->second.bytes);
+        if (it == g_pool_blocks.end()) {
+            drop.push_back(p);
+        } else {
+            const PoolBlock b = it->second;
             g_pool_blocks.erase(it);
+            if (b.array) {
+                array_keep(b.pool, p, b.bytes, &drop);
+            } else {
+                pool = b.pool;
+                pool_use(pool, pool->live - b.bytes);
+            }
         }
     }
     if (pool) cudaFreeAsync(p, pool->stream);
-    else cudaFree(p);
+    for (void* d : drop) cudaFree(d);
 }
 
 // Waits for all work on device `dev`; false when that was refused (while a
@@ -926,7 +1022,7 @@ b2sr_status b2sr_pack_csr(const int* d_rowptr, const int* d_colind, int nrows, i
     m->owns = true;
     b2sr_status st = B2SR_SUCCESS;
     do {
-        m->rowptr = static_cast<int*>(dev_alloc(sizeof(int) * ((size_t)m->nb + 1)));
+        m->rowptr = static_cast<int*>(array_alloc(sizeof(int) * ((size_t)m->nb + 1)));
         if (!m->rowptr) { st = B2SR_ERR_ALLOC; break; }
         PackJob job;
         int nt = 0;
@@ -935,8 +1031,8 @@ b2sr_status b2sr_pack_csr(const int* d_rowptr, const int* d_colind, int nrows, i
         m->nt = nt;
         // the fill writes every colind and tile word; only the padding is zeroed
         const size_t cbytes = sizeof(int) * (size_t)nt, tbytes = (size_t)nt * tile_dim * word_bytes(tile_dim);
-        m->colind = static_cast<int*>(dev_alloc(padded_bytes(cbytes)));
-        m->tiles = dev_alloc(padded_bytes(tbytes));
+        m->colind = static_cast<int*>(array_alloc(padded_bytes(cbytes)));
+        m->tiles = array_alloc(padded_bytes(tbytes));
         if (!m->colind || !m->tiles) { st = B2SR_ERR_ALLOC; break; }
         cudaError_t e = cudaMemsetAsync(reinterpret_cast<char*>(m->colind) + cbytes, 0, padded_bytes(cbytes) - cbytes, s);
         if (e == cudaSuccess)
@@ -1016,12 +1112,14 @@ void b2sr_free(b2sr_matrix* m) {
 
 void b2sr_trim(void) {
     release_matrices({});
-    std::lock_guard<std::mutex> lk(g_pool_mu);
-    for (DevPool& p : g_pools)
-        if (p.pool) {
-            cudaStreamSynchronize(p.stream);
-            cudaMemPoolTrimTo(p.pool, 0);
+    for (int dev = 0; dev < MAX_POOLS; ++dev) {
+        bool made;
+        {
+            std::lock_guard<std::mutex> lk(g_pool_mu);
+            made = g_pools[dev].pool != nullptr;
         }
+        if (made) pool_trim(&g_pools[dev]);
+    }
 }
 
 b2sr_status b2sr_matrix_download(const b2sr_matrix* m, int* h_rowptr, int* h_colind, void* h_tiles) {
@@ -1136,9 +1234,9 @@ b2sr_status b2sr_matrix_load(const char* path, void* stream, b2sr_matrix** out) 
     m->nt = h.nt;
     const size_t cbytes = padded_bytes(sizeof(int) * (size_t)h.nt);
     const size_t tbytes = padded_bytes(tl.size());
-    m->rowptr = static_cast<int*>(dev_alloc(sizeof(int) * rp.size()));
-    m->colind = static_cast<int*>(dev_alloc(cbytes));
-    m->tiles = dev_alloc(tbytes);
+    m->rowptr = static_cast<int*>(array_alloc(sizeof(int) * rp.size()));
+    m->colind = static_cast<int*>(array_alloc(cbytes));
+    m->tiles = array_alloc(tbytes);
     b2sr_status st = B2SR_SUCCESS;
     if (!m->rowptr || !m->colind || !m->tiles) st = B2SR_ERR_ALLOC;
     cudaError_t e = cudaSuccess;
@@ -1187,11 +1285,11 @@ b2sr_status b2sr_matrix_transpose(b2sr_matrix* m, void* stream, const b2sr_matri
     b2sr_status st = B2SR_SUCCESS;
     do {
         t->nt = nt;
-        t->rowptr = static_cast<int*>(dev_alloc(sizeof(int) * ((size_t)t->nb + 1)));
+        t->rowptr = static_cast<int*>(array_alloc(sizeof(int) * ((size_t)t->nb + 1)));
         const size_t cbytes = padded_bytes(sizeof(int) * (size_t)nt);
         const size_t tbytes = padded_bytes((size_t)nt * T * word_bytes(T));
-        t->colind = static_cast<int*>(dev_alloc(cbytes));
-        t->tiles = dev_alloc(tbytes);
+        t->colind = static_cast<int*>(array_alloc(cbytes));
+        t->tiles = array_alloc(tbytes);
         if (!t->rowptr || !t->colind || !t->tiles) { st = B2SR_ERR_ALLOC; break; }
         cudaError_t e = cudaMemsetAsync(t->colind, 0, cbytes, s);
         if (e == cudaSuccess) e = cudaMemsetAsync(t->tiles, 0, tbytes, s);

@@ -136,6 +136,7 @@ namespace b2sr {
 // ---- status / allocation helpers (b2sr_api.cu) --------------------------------
 void set_cuda_error(cudaError_t e);
 void* dev_alloc(size_t bytes);
+void* array_alloc(size_t bytes);  // for a matrix's arrays: a block of cudaMalloc (no hook); freed by dev_free
 void dev_free(void* p);
 void set_launch_count(int n);
 void add_launch_count(int n);

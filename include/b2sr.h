@@ -121,6 +121,9 @@ b2sr_status b2sr_matrix_wrap(const int* d_rowptr, const int* d_colind, const voi
  * B2SR_ERR_INVALID_VALUE: a tile-column of `m` outside the matrix. */
 b2sr_status b2sr_matrix_transpose(b2sr_matrix* m, void* stream, const b2sr_matrix** out_t);
 
+/* Without an allocation hook the arrays of a packed, loaded or transposed matrix
+ * are blocks of cudaMalloc, each its own: cudaIpcGetMemHandle takes them and
+ * cudaDeviceEnablePeerAccess opens them. */
 b2sr_status b2sr_matrix_describe(const b2sr_matrix* m, b2sr_matrix_desc* out);
 /* Waits for the device, then frees the matrix.  While a stream is being captured
  * that wait is refused (and, as CUDA has it, the capture is invalidated): the
