@@ -17,6 +17,15 @@ def pytest_configure(config):
     config.addinivalue_line("markers", "gpu: needs a CUDA GPU (runs the CUDA kernels)")
 
 
+# Need what is built from the reference's checkout and fail where it is absent: a run that stops at the
+# first failure has then run everything else.
+REFERENCE_FILES = {"test_gpu_ref_drivers.py", "test_gpu_reference_kernels.py", "test_gpu_reference_speed.py"}
+
+
+def pytest_collection_modifyitems(items):
+    items.sort(key=lambda item: item.path.name in REFERENCE_FILES)
+
+
 @pytest.fixture(scope="session")
 def built():
     entry.build()
