@@ -49,7 +49,7 @@ static void* g_alloc_ctx = nullptr;
 
 // ---- device memory ---------------------------------------------------------------
 // Without a caller's allocator, device memory comes from two places per device.
-// Each keeps up to 1/512 of the device's memory (0.55 GB on GB300) that was
+// Each keeps up to 1/256 of the device's memory (1.1 GB on GB300) that was
 // freed; all of it goes back on b2sr_trim and before an allocation fails.
 // cudaMalloc takes 40 - 80 us and cudaFree 30 - 110 us on GB300; packing a graph,
 // transposing it and building its plans makes some 50 such calls.
@@ -116,7 +116,7 @@ DevPool* device_pool(int dev) {
                   cudaStreamCreateWithFlags(&p.stream, cudaStreamNonBlocking) == cudaSuccess &&
                   cudaMemPoolCreate(&p.pool, &props) == cudaSuccess;
         if (ok) {
-            p.keep = prop.totalGlobalMem / 512;
+            p.keep = prop.totalGlobalMem / 256;
             ok = pool_use(&p, 0) == cudaSuccess;
         }
         if (!ok) {
@@ -162,13 +162,13 @@ cudaError_t malloc_relaxed(void** p, size_t bytes) {
     return e;
 }
 
-// An array of at least *bytes; *bytes becomes its size: rounded up to an eighth
-// of a power of two where it may be kept, so that arrays of about the same size
-// (a graph per step) take each other's blocks.
+// An array of at least *bytes; *bytes becomes its size: where it may be kept,
+// rounded up to an eighth of a power of two (a 64th above 16 MB), so that arrays
+// of about the same size (a graph per step) take each other's blocks.
 cudaError_t array_take(DevPool* pool, void** p, size_t* bytes) {
     if (*bytes <= pool->keep) {
         size_t step = 512;
-        while (step * 16 <= *bytes) step *= 2;
+        while (step * (*bytes <= ((size_t)16 << 20) ? 16 : 128) <= *bytes) step *= 2;
         *bytes = (*bytes + step - 1) / step * step;
         std::lock_guard<std::mutex> lk(g_pool_mu);
         auto best = pool->arrays.end();

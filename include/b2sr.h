@@ -91,7 +91,7 @@ typedef void* (*b2sr_alloc_fn)(size_t bytes, void* ctx);
 typedef void (*b2sr_free_fn)(void* ptr, void* ctx);
 void b2sr_set_allocator(b2sr_alloc_fn alloc_fn, b2sr_free_fn free_fn, void* ctx);
 
-/* Without a hook the library keeps up to 1/256 of a device's memory that it has
+/* Without a hook the library keeps up to 1/128 of a device's memory that it has
  * freed, for its next allocations.  b2sr_trim gives all of it back to the
  * driver (so does an allocation that would otherwise fail). */
 void b2sr_trim(void);
