@@ -64,8 +64,8 @@ struct RowBinPlan {
     int warp_off[7] = {0, 0, 0, 0, 0, 0, 0};
 };
 
-// Row-task SpMM plan (b2sr_spmm_rows.cu, T = 4 and 8): one task per
-// tile-row in row order, long rows cut into segments with partial slots.
+// Row-task SpMM plan (b2sr_spmm_rows.cu): one task per tile-row, long ones cut
+// into segments with partial slots; larger tasks first.
 struct SpmmRowsPlan {
     int4* d_tasks = nullptr;
     int4* d_long = nullptr;      // (tile-row, first slot, slots, 0)
@@ -101,7 +101,7 @@ struct b2sr_matrix {
     bool rowbin_ready = false;
     b2sr::RowBinPlan rowbin_bits;  // the bit-vector kernels' plan
     bool rowbin_bits_ready = false;
-    b2sr::SpmmRowsPlan spmm_rows;  // row-task SpMM plan (T = 4, 8)
+    b2sr::SpmmRowsPlan spmm_rows;  // row-task SpMM plan
     bool spmm_rows_ready = false;
     // Held while a call launches its kernels: they share the stream's scratch, so
     // those of two host threads on one stream must not come in between.
@@ -235,11 +235,10 @@ constexpr int PLAN_CLASSES = 64;
 //   BINS    nbins bins by tile count (bin b: up to unit << b tiles), the last
 //           bin first
 //   TWO     tasks of at least a quarter of seg, then the rest
-//   LENGTH  longest first, in four classes per octave
 //   BITS    most set bits first, in two classes per octave
 // Long rows of at most narrow_slots slots are listed before the others.
 struct PlanRule {
-    enum Kind { BINS, TWO, LENGTH, BITS } kind;
+    enum Kind { BINS, TWO, BITS } kind;
     int seg;
     int classes;
     int unit = 0, nbins = 0, narrow_slots = 0;

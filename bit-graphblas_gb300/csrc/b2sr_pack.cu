@@ -120,7 +120,7 @@ __host__ __device__ __forceinline__ int chunks_of(int entries, int T) {
     return entries == 0 ? 0 : entries <= CHUNK_CAP ? 1 : (entries + per - 1) / per;
 }
 
-// Chunks of every tile-row, and their sums per SCAN_TILE tile-rows.
+// Chunks of every tile-row.
 __global__ void chunk_plan_kernel(const int* __restrict__ rowptr, int nrows, int nb, int T,
                                   const PackInfo* __restrict__ info, int* __restrict__ nch) {
     const long long tr = blockIdx.x * (long long)blockDim.x + threadIdx.x;

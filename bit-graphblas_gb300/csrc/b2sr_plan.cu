@@ -31,13 +31,12 @@ struct RowTasks {
     bool narrow; // long row listed before the others
 };
 
-// Size classes, largest first: PER per octave.
-template <int PER>
+// Size classes, largest first: two per octave.
 __device__ __forceinline__ int size_class(long long v) {
     if (v <= 0) return PLAN_CLASSES - 1;
     const int e = 63 - __clzll(v);
-    const int sub = PER == 4 ? (e >= 2 ? (int)(v >> (e - 2)) & 3 : (int)(v << (2 - e)) & 3) : (e >= 1 ? (int)(v >> (e - 1)) & 1 : 0);
-    return max(PLAN_CLASSES - 1 - (PER * e + sub), 0);
+    const int sub = e >= 1 ? (int)(v >> (e - 1)) & 1 : 0;
+    return max(PLAN_CLASSES - 1 - (2 * e + sub), 0);
 }
 
 __device__ __forceinline__ RowTasks row_tasks(const PlanRule& r, const int* __restrict__ rowptr, int i, int nb) {
@@ -62,8 +61,7 @@ __device__ __forceinline__ RowTasks row_tasks(const PlanRule& r, const int* __re
     t.narrow = t.nseg <= r.narrow_slots;
     const int len = (t.m + t.nseg - 1) / t.nseg;  // of a segment
     if (r.kind == PlanRule::TWO) t.cls = 4LL * len >= r.seg ? 0 : 1;
-    else if (r.kind == PlanRule::LENGTH) t.cls = size_class<4>(len);
-    else t.cls = size_class<2>(bits / t.nseg);
+    else t.cls = size_class(bits / t.nseg);
     return t;
 }
 

@@ -882,9 +882,10 @@ __device__ __forceinline__ void wide_bits_rows(const RowBinBitsArgs& a, int task
     for (int p = 0; p < 2; ++p) wide_bits_group<T, KIND, G>(a, task0 + p * (WIDE_PASS<T> / G), tend, skip);
 }
 
-// T <= 16 fits 32 registers: 64 warps per SM.  At T = 16 on R-MAT scale 20 the
-// bit kinds (no spills) take 121.5 instead of 133.1 us at 40 registers, the
-// count kinds (a few spills) 124.9 instead of 128.6.  T = 32 fits 40: 48 warps.
+// T <= 16 fits 32 registers without spills: 64 warps per SM.  At T = 16 on R-MAT
+// scale 20 the bit kinds take 105 us and the count kinds 116 (40 registers, with
+// the row tests of that time: 133.1 instead of 121.5, and 128.6 instead of
+// 124.9).  T = 32 fits 40: 48 warps.
 template <int T, int KIND>
 __global__ void __launch_bounds__(256, T <= 8 ? 8 : 1) __maxnreg__((T == 32 ? 40 : T == 16 ? 32 : 255))
     rowbin_bits_kernel(RowBinBitsArgs a) {

@@ -3,11 +3,12 @@
 // dX = A^T . dY is the same kernel on the transposed B2SR).  A work item is one
 // group of 4 rows of a task, T/4 items per task and column block.
 //
-// Plan (once per matrix, b2sr_plan.cu): one task per tile-row; a tile-row
-// longer than spmm_rows_seg() tiles (a share of one resident warp's part of all
-// the tiles), or at T >= 8 with more than such a share of the set bits, is cut
-// into near-equal segments whose partial rows go to slots, which a second
-// kernel adds in segment order.  Warps take
+// Plan (once per matrix, b2sr_plan.cu): one task per tile-row.  A tile-row of
+// more than rows_whole_tiles() tiles that is longer than spmm_rows_seg() tiles (a
+// share of one resident warp's part of all the tiles), or at T >= 8 one of more
+// than ROWS_WHOLE_BITS set bits and more than such a share of them, is cut into
+// near-equal segments whose partial rows go to slots, which a second kernel adds
+// in segment order.  Warps take
 // (column block, task, row group) work items from a device queue (an atomic
 // counter); long tasks are handed out first, so the queue ends on short ones
 // (R-MAT hubs sit all over the vertex range, and in row order the last items

@@ -15,14 +15,14 @@
 // Sums visit a row's tiles in a fixed order, so they are reproducible.
 //
 // GB300, R-MAT scale 20 unless said otherwise, lane per tile -> this form:
-//   T = 32 bin_bin_bin 1% / 30% frontier   419 / 419 -> 205 / 273 us
-//   T = 32 int32 counts, 30%               525 -> 298 us
+//   T = 32 bin_bin_bin 1% / 30% frontier   419 / 419 -> 194 / 276 us
+//   T = 32 int32 counts, 30%               525 -> 292 us
 //   T = 32 FP32 sums                       673 -> 505 us (2.9 -> 3.9 TB/s of
 //     tiles); 300,000-vertex ER graph of degree 16: 178 -> 135 us
 //   64 frontiers, R-MAT scale 18: T = 32 723 -> 174 us, T = 16 287 -> 144 us;
 //   32 frontiers: 403 -> 130 us, 148 -> 91 us
-// Bit vectors at T = 16 stay with a lane per tile (112 us; 138 us this way: a
-// lane's two 16-byte loads already use every sector they touch).
+// Bit vectors at T = 16 stay with a lane per tile (112 us when this was 138; 105
+// now: a lane's two 16-byte loads already use every sector they touch).
 #pragma once
 
 #include "b2sr_spmv_impl.cuh"

@@ -102,8 +102,9 @@ void b2sr_trim(void);
  * Replaces CSR2HSBSF (bmv_eval/test_bin_full_full.cu:167-211) = cusparseXcsr2bsrNnz
  * + csr2bsr_batch_{T} (bmv_eval/backend/csr2bsr_batch_bsrbmv.cu:16,140,263,386).
  * The CSR is validated on the device first; a bad CSR returns
- * B2SR_ERR_INVALID_CSR and packs nothing.  Synchronises `stream` once (the tile
- * count decides the allocation size). */
+ * B2SR_ERR_INVALID_CSR and packs nothing (no column is read unless the row
+ * pointer is good).  Synchronises `stream` (the tile count decides the allocation
+ * size; the matrix is complete on return). */
 b2sr_status b2sr_pack_csr(const int* d_rowptr, const int* d_colind, int nrows, int ncols,
                           int nnz, int tile_dim, void* stream, b2sr_matrix** out);
 
