@@ -857,15 +857,22 @@ static void free_matrix(b2sr_matrix* m) {
 static std::mutex g_unfreed_mu;
 static std::vector<b2sr_matrix*> g_unfreed;
 static void release_matrices(std::vector<b2sr_matrix*> drop) {
-    std::lock_guard<std::mutex> lk(g_unfreed_mu);
-    drop.insert(drop.end(), g_unfreed.begin(), g_unfreed.end());
-    g_unfreed.clear();
+    {
+        std::lock_guard<std::mutex> lk(g_unfreed_mu);
+        drop.insert(drop.end(), g_unfreed.begin(), g_unfreed.end());
+        g_unfreed.clear();
+    }
+    // no lock from here: a caller's free_fn may come back to free another matrix
     int dev = -1;
     bool idle = false;
     for (b2sr_matrix* m : drop) {
         if (m->device != dev) idle = sync_device(dev = m->device);
-        if (idle) free_matrix(m);
-        else g_unfreed.push_back(m);
+        if (idle) {
+            free_matrix(m);
+        } else {
+            std::lock_guard<std::mutex> lk(g_unfreed_mu);
+            g_unfreed.push_back(m);
+        }
     }
 }
 

@@ -121,3 +121,21 @@ def test_free_during_a_capture_keeps_the_memory(pkg, cuda, later):
         assert h.freed > 0
         B.close()
         assert not h.blocks
+
+
+def test_a_free_hook_may_free_another_matrix(pkg, cuda):
+    """As Python's garbage collector does, when it runs inside the hook."""
+    g = pkg.erdos_renyi(1000, 4.0, seed=1)
+    with hooked(pkg) as h:
+        A, B = pkg.B2SRMatrix.from_graph(g, 8, device=cuda), pkg.B2SRMatrix.from_graph(g, 4, device=cuda)
+        others = [B]
+
+        class Blocks(dict):
+            def pop(self, ptr):
+                if others:
+                    others.pop().close()
+                return super().pop(ptr)
+
+        h.blocks = Blocks(h.blocks)
+        A.close()
+        assert not h.blocks
